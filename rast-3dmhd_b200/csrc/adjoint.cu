@@ -7,12 +7,11 @@
 // segment from its checkpoint, then for each step (last first) recomputes the three stages
 // once more - now also storing the right-hand sides F_s (stage kernels with EMIT) - and runs
 //
-//   for s = 2, 1, 0:   lambda_Y   = BCON^T lambda_X_{s+1}            (adj_bcon_kernel)
-//                      lambda_F_s += gam_s dt lambda_Y               (adj_seed_kernel)
-//                      lambda_X_s  = F'(X_s)^T lambda_F_s + lambda_Y (adj_pass1/pass2_kernel)
-//                      lambda_F_{s-1} = zeta_s dt lambda_Y
-//   lambda_dt = sum_s gam_s <F_s, lambda_Y> + zeta_s <F_{s-1}, lambda_Y>   (deterministic sum)
-//   lambda_X_0 += lambda_dt * sff * d(limit)/dX at the cell that set dt (adj_argmin, adj_dt)
+//   for s = 2, 1, 0:   lambda_Y   = BCON^T lambda_X_{s+1}                       (adj_bcon_kernel)
+//                      lambda_F_s = gam_s dt lambda_Y + zeta_{s+1} dt lambda_Y(s+1)  (adj_pass1_kernel)
+//                      lambda_X_s = F'(X_s)^T lambda_F_s + lambda_Y             (adj_pass2_kernel)
+//   lambda_dt = sum_s <F_s, lambda_F_s> / dt                                    (deterministic sum)
+//   lambda_X_0 += lambda_dt * sff * d(limit)/dX at the cell that set dt (dt_argmin_kernel, adj_dt_apply)
 //
 // Each recomputed step is compared bit for bit with the recorded state that follows it; a
 // mismatch (a non-reproducible forward) is reported as R3D_ENUMERIC instead of a silently wrong
@@ -33,16 +32,14 @@ using r3dk::AdjArgs;
 
 namespace {
 
-constexpr int kDots = 5;  // gam_2, gam_1, gam_0 dots (seed) and zeta_2, zeta_1 dots (pass 2)
-constexpr int BX = 32, BY = 4;
+constexpr int BX = 32, BY = 8;       // cells per block of the passes
+constexpr int kDotBlocks = 32;        // partial sums of the dt dot products
 
 struct AdjScalars {
     unsigned long long wkey[4];  // the step's four limit minima (ordered keys), saved before dt
     unsigned long long argmin;   // smallest cell index holding the winning limit
     unsigned long long mismatch; // recompute vs recorded state: differing values
-    double lam_dt;
-    double mstar;
-    int term;
+    double part[kDotBlocks];     // partial sums of <F_s, lambda_F_s> over the three stages
 };
 
 __device__ __forceinline__ int block_linear() {
@@ -63,130 +60,84 @@ __device__ void block_sum_store(double v, double* out) {
     }
 }
 
+struct FieldPtrs {
+    const double* x[r3dk::kMaxFields];
+    double* lam[r3dk::kMaxFields];
+};
+
 __global__ void __launch_bounds__(BX* BY) adj_bcon_kernel(r3dk::Geometry g, r3dk::Physics ph,
-                                                           r3dk::Boundary bd, AdjArgs A) {
+                                                           r3dk::Boundary bd, FieldPtrs A, int nf) {
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
     if (i > g.npx || j > g.npy) return;
-    r3dk::adj_bcon_column(g, ph, bd, A.x, A.lam, A.nf, i, j);
+    // one side per thread, or (npz < 6: the two sides share planes) both in turn
+    const int z = blockIdx.z;
+    r3dk::adj_bcon_column(g, ph, bd, A.x, A.lam, nf, z, i, j);
+    if (gridDim.z == 1) r3dk::adj_bcon_column(g, ph, bd, A.x, A.lam, nf, 1, i, j);
 }
 
-// lambda_F (+)= gam dt lambda_Y on the interior; partial dot <F_s, lambda_Y> per block.
-__global__ void __launch_bounds__(BX* BY) adj_seed_kernel(AdjArgs A, double* lamF0, double* lamF1, double* lamF2,
-                                                           double* lamF3, double* lamF4, double* lamF5,
-                                                           double* lamF6, double* lamF7, double gam, int first,
-                                                           double* dots) {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+// Bound by the latency of the gathers, so by how many loads the warps of an SM keep in flight: two
+// 256-thread blocks per SM (three for hydro pass 1) with every load of a cell free to go out at once.
+// B200, us per stage: 128x128x128 hydro pass 1 154 (two blocks: 165), pass 2 170 (three blocks, 80
+// registers and spills: 192); 64x64x128 MHD pass 1 69 (three: 77), pass 2 87 (three: 97).  The passes
+// they replace, which stored every Lambda and folded lambda_F separately: 577 and 222.
+template <bool MHD>
+__global__ void __launch_bounds__(BX* BY, MHD ? 2 : 3) adj_pass1_kernel(const __grid_constant__ AdjArgs A, double* dots) {
+    const int i = 1 + blockIdx.x * BX + threadIdx.x;
+    const int j = 1 + blockIdx.y * BY + threadIdx.y;
     const int k = 1 + blockIdx.z;
-    double* lf[8] = {lamF0, lamF1, lamF2, lamF3, lamF4, lamF5, lamF6, lamF7};
     double dot = 0.0;
-    if (i <= A.g.npx && j <= A.g.npy) {
-        const int n = k * (int)A.g.plane + j * (int)A.g.pitch + i;
-        const double gdt = gam * A.sc->dt;
-#pragma unroll
-        for (int f = 0; f < 8; ++f) {  // unrolled: the pointer table stays in registers
-            if (f < A.nf) {
-                const double ly = A.lam[f][n];
-                lf[f][n] = (first ? 0.0 : lf[f][n]) + gdt * ly;
-                dot += A.fprev[f][n] * ly;  // fprev carries F_s here
-            }
-        }
-    }
+    if (i <= A.g.npx && j <= A.g.npy) dot = r3dk::adj_pass1_cell<MHD>(A, i, j, k);
     block_sum_store(dot, dots);
 }
 
-__global__ void __launch_bounds__(BX* BY) adj_pass1_kernel(AdjArgs A) {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+template <bool MHD>
+__global__ void __launch_bounds__(BX* BY, 2) adj_pass2_kernel(const __grid_constant__ AdjArgs A) {
+    const int i = 1 + blockIdx.x * BX + threadIdx.x;
+    const int j = 1 + blockIdx.y * BY + threadIdx.y;
     const int k = 1 + blockIdx.z;
-    if (i <= A.g.npx && j <= A.g.npy) r3dk::adj_pass1_cell(A, i, j, k);
-}
-
-__global__ void __launch_bounds__(BX* BY) adj_pass2_kernel(AdjArgs A, double* dots) {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = 1 + blockIdx.z;
-    double dot = 0.0;
-    if (i <= A.g.npx && j <= A.g.npy) dot = r3dk::adj_pass2_cell(A, i, j, k);
-    if (dots) block_sum_store(dot, dots);
+    if (i <= A.g.npx && j <= A.g.npy) r3dk::adj_pass2_cell<MHD>(A, i, j, k);
 }
 
 __global__ void adj_save_limits_kernel(const r3dk::Scalars* sc, AdjScalars* aux) {
     for (int q = 0; q < 4; ++q) aux->wkey[q] = sc->wmin[q];
+    aux->argmin = ~0ull;
 }
 
-// lambda_dt from the five dot products (fixed summation order), and the winning limit as
-// step_begin_kernel chooses it.
-// One block of kSumThreads: a fixed summation order (deterministic), many loads in flight.
-constexpr int kSumThreads = 1024;
-__global__ void __launch_bounds__(kSumThreads) adj_dt_sum_kernel(r3dk::Physics ph, const double* dots, int nblocks,
-                                                                  double c0, double c1, double c2, double c3,
-                                                                  double c4, AdjScalars* aux) {
+// The n dot-product partials of the step's passes to kDotBlocks sums, each over a fixed share in
+// a fixed order (deterministic).  One block summing all of them took 41 us at 128x128x128.
+constexpr int kSumThreads = 256;
+__global__ void __launch_bounds__(kSumThreads) adj_dots_kernel(const double* dots, int n, AdjScalars* aux) {
     __shared__ double red[kSumThreads];
-    const double coef[kDots] = {c0, c1, c2, c3, c4};
     double s = 0.0;
-    for (int d = 0; d < kDots; ++d) {
-        double p = 0.0;
-        for (int b = threadIdx.x; b < nblocks; b += blockDim.x) p += dots[(size_t)d * nblocks + b];
-        s += coef[d] * p;
-    }
+    for (int b = blockIdx.x * kSumThreads + threadIdx.x; b < n; b += kDotBlocks * kSumThreads) s += dots[b];
     red[threadIdx.x] = s;
     __syncthreads();
     for (int w = kSumThreads / 2; w > 0; w >>= 1) {
         if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        aux->lam_dt = red[0];
-        const double w0 = r3dk::order_value(aux->wkey[0]), w1 = r3dk::order_value(aux->wkey[1]);
-        const double w2 = r3dk::order_value(aux->wkey[2]), w3 = r3dk::order_value(aux->wkey[3]);
-        int t = 0;
-        double m = w0;
-        if (w1 < m) { t = 1; m = w1; }
-        if (w2 < m) { t = 2; m = w2; }
-        if (ph.lmag && w3 < m) { t = 3; m = w3; }
-        aux->term = t;
-        aux->mstar = m;
-        aux->argmin = ~0ull;
-    }
+    if (threadIdx.x == 0) aux->part[blockIdx.x] = red[0];
 }
 
-__global__ void __launch_bounds__(BX* BY) adj_argmin_kernel(r3dk::Geometry g, r3dk::Physics ph, r3dk::Lines L,
-                                                             AdjArgs A, AdjScalars* aux) {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = 1 + blockIdx.z;
-    if (i > g.npx || j > g.npy) return;
-    const int term = aux->term;
-    if (term == 3) return;  // the constant magnetic-diffusion limit has no derivative
-    const int n = k * (int)g.plane + j * (int)g.pitch + i;
-    double b2 = 0.0;
-    if (ph.lmag) {
-        const double bx = A.x[5][n], by = A.x[6][n], bz = A.x[7][n];
-        b2 = bx * bx + by * by + bz * bz;
-    }
-    const double dxy = (L.ddy[j] < L.ddx[i]) ? L.ddy[j] : L.ddx[i];
-    const double dd = (L.ddz[k] < dxy) ? L.ddz[k] : dxy;  // the dt_full_kernel expression
-    double w1, w2, w3, w4, um;
-    r3dk::dt_terms(ph, A.x[0][n], A.x[1][n], A.x[2][n], A.x[3][n], A.x[4][n], b2, dd, L.rkapa[k], w1, w2, w3,
-                   w4, um);
-    const double wq = term == 0 ? w1 : (term == 1 ? w2 : w3);
-    if (wq == aux->mstar) atomicMin(&aux->argmin, (unsigned long long)n);
-}
-
-__global__ void adj_dt_apply_kernel(r3dk::Geometry g, r3dk::Physics ph, r3dk::Lines L, AdjArgs A,
-                                    AdjScalars* aux) {
+// lambda_X_0 += lambda_dt * sff * d(limit)/dX at the cell that set dt.
+__global__ void adj_dt_apply_kernel(r3dk::Geometry g, r3dk::Physics ph, r3dk::Lines L, const double* x, double* lam,
+                                    int64_t fe, int nf, const r3dk::Scalars* sc, const AdjScalars* aux) {
     const unsigned long long an = aux->argmin;
-    if (aux->term == 3 || an == ~0ull) return;
+    double mstar;
+    const int term = r3dk::winning_limit(aux->wkey, ph.lmag, mstar);
+    if (term == 3 || an == ~0ull) return;
+    double lam_dt = 0.0;
+    for (int b = 0; b < kDotBlocks; ++b) lam_dt += aux->part[b];
+    lam_dt /= sc->dt;
     const int n = (int)an;
     const int k = n / (int)g.plane, j = (n % (int)g.plane) / (int)g.pitch, i = n % (int)g.pitch;
     const double dxy = (L.ddy[j] < L.ddx[i]) ? L.ddy[j] : L.ddx[i];
     const double dd = (L.ddz[k] < dxy) ? L.ddz[k] : dxy;
     double xv[r3dk::kMaxFields], gv[r3dk::kMaxFields];
-    for (int f = 0; f < A.nf; ++f) xv[f] = A.x[f][n];
-    r3dk::adj_dt_cell(ph, aux->term, dd, L.rkapa[k], xv, A.nf, aux->lam_dt * ph.sff, gv);
-    for (int f = 0; f < A.nf; ++f) A.lam[f][n] += gv[f];
+    for (int f = 0; f < nf; ++f) xv[f] = x[f * fe + n];
+    r3dk::adj_dt_cell(ph, term, dd, L.rkapa[k], xv, nf, lam_dt * ph.sff, gv);
+    for (int f = 0; f < nf; ++f) lam[f * fe + n] += gv[f];
 }
 
 // Count interior values that differ (bitwise) between a recomputed and a recorded state.
@@ -219,10 +170,11 @@ struct Adjoint {
     StateBuf S[4];                  // X_0 .. X_3 of the step being reversed
     double* Zb = nullptr;           // accumulator Z (nf fields)
     double* F[3] = {};              // F_0 .. F_2 (nf fields each)
-    double* lam = nullptr;          // lambda_X (nf fields)
-    double* lamF[2] = {};           // lambda_F, two buffers
-    double* Lam = nullptr;          // pass-1 arrays
-    int nlam = 0;
+    double* lam[2] = {};            // lambda_X / lambda_Y of a stage and of the one after it
+    int cur = 0;                    // lam[cur] is the current one
+    double* a = nullptr;            // lambda_F (nf fields)
+    double* mid = nullptr;          // pass-1 arrays
+    int nmid = 0;
     double* dots = nullptr;
     int nblocks = 0;
     r3dk::Scalars* asc = nullptr;   // scalars of the recompute
@@ -276,23 +228,23 @@ Adjoint* workspace(r3d_gpu* g) {
         }
         A->Zb = dalloc(A, st);
         for (int s = 0; s < 3; ++s) A->F[s] = dalloc(A, st);
-        A->lam = dalloc(A, st);
-        for (int s = 0; s < 2; ++s) A->lamF[s] = dalloc(A, st);
-        A->nlam = A->nf == 8 ? r3dk::kLamMax : r3dk::kLamHydro;
-        A->Lam = dalloc(A, (size_t)A->nlam * A->field_elems);
+        for (int s = 0; s < 2; ++s) A->lam[s] = dalloc(A, st);
+        A->a = dalloc(A, st);
+        A->nmid = A->nf == 8 ? r3dk::kMidMax : r3dk::kMidHydro;
+        A->mid = dalloc(A, (size_t)A->nmid * A->field_elems);
         const dim3 gr = cell_grid(g);
         A->nblocks = (int)(gr.x * gr.y * gr.z);
-        A->dots = dalloc(A, (size_t)kDots * A->nblocks);
+        A->dots = dalloc(A, (size_t)3 * A->nblocks);
         cuda_ok(cudaMalloc(&A->asc, sizeof(r3dk::Scalars)), "cudaMalloc(adjoint scalars)");
         cuda_ok(cudaMemsetAsync(A->asc, 0, sizeof(r3dk::Scalars), g->stream), "cudaMemset");
         cuda_ok(cudaMalloc(&A->aux, sizeof(AdjScalars)), "cudaMalloc(adjoint scalars)");
         cuda_ok(cudaMemsetAsync(A->aux, 0, sizeof(AdjScalars), g->stream), "cudaMemset");
         cuda_ok(cudaMallocHost(&A->haux, sizeof(AdjScalars)), "cudaMallocHost");
-        // F, Lambda and the lambda buffers are read at ghost-free interior cells only, but keep
-        // every buffer defined
-        for (double* p : {A->Zb, A->F[0], A->F[1], A->F[2], A->lam, A->lamF[0], A->lamF[1]})
+        // the z ghost planes of a and mid are read (with weight 0) and stay zero; keep every
+        // other buffer defined as well
+        for (double* p : {A->Zb, A->F[0], A->F[1], A->F[2], A->lam[0], A->lam[1], A->a})
             cuda_ok(cudaMemsetAsync(p, 0, st * sizeof(double), g->stream), "cudaMemset");
-        cuda_ok(cudaMemsetAsync(A->Lam, 0, (size_t)A->nlam * A->field_elems * sizeof(double), g->stream),
+        cuda_ok(cudaMemsetAsync(A->mid, 0, (size_t)A->nmid * A->field_elems * sizeof(double), g->stream),
                 "cudaMemset");
     } catch (...) {
         g->adj = A;
@@ -353,63 +305,52 @@ void recompute_step(r3d_gpu* g, Adjoint* A, const double* src) {
     }
 }
 
-AdjArgs base_args(const r3d_gpu* g, const Adjoint* A) {
-    AdjArgs a{};
-    a.g = g->geo;
-    a.ph = g->ph;
-    a.L = g->lines;
-    a.nf = A->nf;
-    a.sc = A->asc;
-    for (int q = 0; q < A->nlam; ++q) a.Lam[q] = A->Lam + (size_t)q * A->field_elems;
-    for (int f = 0; f < A->nf; ++f) a.lam[f] = state_field(A->lam, A, f);
-    return a;
-}
-
-// Reverse the step whose intermediates recompute_step left in the workspace: lam holds the
+// Reverse the step whose intermediates recompute_step left in the workspace: lam[cur] holds the
 // adjoint of X_3 on entry and of X_0 on exit.
 void reverse_step(r3d_gpu* g, Adjoint* A) {
     const dim3 blk(BX, BY, 1), cg = cell_grid(g);
-    const dim3 cols((g->geo.npx + BX - 1) / BX, (g->geo.npy + BY - 1) / BY, 1);
-    const double gam[3] = {g->ph.gam[0], g->ph.gam[1], g->ph.gam[2]};
-    const double zeta[3] = {g->ph.zeta[0], g->ph.zeta[1], g->ph.zeta[2]};
-    int cur = 0;
+    const dim3 cols(cg.x, cg.y, g->geo.npz < 6 ? 1 : 2);
+    const bool mhd = A->nf == 8;
     for (int s = 2; s >= 0; --s) {
-        AdjArgs a = base_args(g, A);
-        for (int f = 0; f < A->nf; ++f) a.x[f] = state_field(A->S[s + 1].base, A, f);
-        adj_bcon_kernel<<<cols, blk, 0, g->stream>>>(g->geo, g->ph, g->bnd, a);
+        double* lam = A->lam[A->cur];
+        double* other = A->lam[1 - A->cur];  // lambda_Y of stage s + 1, then lambda_X of stage s
+        FieldPtrs fp{};
+        for (int f = 0; f < A->nf; ++f) {
+            fp.x[f] = state_field(A->S[s + 1].base, A, f);
+            fp.lam[f] = state_field(lam, A, f);
+        }
+        adj_bcon_kernel<<<cols, blk, 0, g->stream>>>(g->geo, g->ph, g->bnd, fp, A->nf);
         cuda_ok(cudaGetLastError(), "adj_bcon");
-        double* lf[8] = {};
-        for (int f = 0; f < A->nf; ++f) {
-            lf[f] = state_field(A->lamF[cur], A, f);
-            a.fprev[f] = state_field(A->F[s], A, f);
-        }
-        adj_seed_kernel<<<cg, blk, 0, g->stream>>>(a, lf[0], lf[1], lf[2], lf[3], lf[4], lf[5], lf[6], lf[7],
-                                                   gam[s], s == 2 ? 1 : 0, A->dots + (size_t)(2 - s) * A->nblocks);
-        cuda_ok(cudaGetLastError(), "adj_seed");
-        AdjArgs p = base_args(g, A);
-        for (int f = 0; f < A->nf; ++f) {
-            p.x[f] = state_field(A->S[s].base, A, f);
-            p.a[f] = lf[f];
-            if (s > 0) {
-                p.fnext[f] = state_field(A->lamF[1 - cur], A, f);
-                p.fprev[f] = state_field(A->F[s - 1], A, f);
-            }
-        }
-        p.zeta = zeta[s];
-        adj_pass1_kernel<<<cg, blk, 0, g->stream>>>(p);
+        AdjArgs p{};
+        p.g = g->geo;
+        p.ph = g->ph;
+        p.L = g->lines;
+        p.fe = A->field_elems;
+        p.x = A->S[s].base;
+        p.lam = lam;
+        p.lprev = s < 2 ? other : nullptr;
+        p.a = A->a;
+        p.mid = A->mid;
+        p.out = other;
+        p.F = A->F[s];
+        p.sc = A->asc;
+        p.gam = g->ph.gam[s];
+        p.zeta = s < 2 ? g->ph.zeta[s + 1] : 0.0;
+        double* dots = A->dots + (size_t)s * A->nblocks;
+        if (mhd) adj_pass1_kernel<true><<<cg, blk, 0, g->stream>>>(p, dots);
+        else adj_pass1_kernel<false><<<cg, blk, 0, g->stream>>>(p, dots);
         cuda_ok(cudaGetLastError(), "adj_pass1");
-        adj_pass2_kernel<<<cg, blk, 0, g->stream>>>(p, s > 0 ? A->dots + (size_t)(3 + (2 - s)) * A->nblocks : nullptr);
+        if (mhd) adj_pass2_kernel<true><<<cg, blk, 0, g->stream>>>(p);
+        else adj_pass2_kernel<false><<<cg, blk, 0, g->stream>>>(p);
         cuda_ok(cudaGetLastError(), "adj_pass2");
-        cur = 1 - cur;
+        A->cur = 1 - A->cur;
     }
-    adj_dt_sum_kernel<<<1, kSumThreads, 0, g->stream>>>(g->ph, A->dots, A->nblocks, gam[2], gam[1], gam[0], zeta[2], zeta[1],
-                                               A->aux);
-    cuda_ok(cudaGetLastError(), "adj_dt_sum");
-    AdjArgs d = base_args(g, A);
-    for (int f = 0; f < A->nf; ++f) d.x[f] = state_field(A->S[0].base, A, f);
-    adj_argmin_kernel<<<cg, blk, 0, g->stream>>>(g->geo, g->ph, g->lines, d, A->aux);
-    cuda_ok(cudaGetLastError(), "adj_argmin");
-    adj_dt_apply_kernel<<<1, 1, 0, g->stream>>>(g->geo, g->ph, g->lines, d, A->aux);
+    adj_dots_kernel<<<kDotBlocks, kSumThreads, 0, g->stream>>>(A->dots, 3 * A->nblocks, A->aux);
+    cuda_ok(cudaGetLastError(), "adj_dots");
+    cuda_ok(r3dk::launch_dt_argmin(g->geo, g->ph, g->lines, stage_fields(A, 0), A->aux->wkey, &A->aux->argmin, g->stream),
+            "adj_argmin");
+    adj_dt_apply_kernel<<<1, 1, 0, g->stream>>>(g->geo, g->ph, g->lines, A->S[0].base, A->lam[A->cur], A->field_elems,
+                                               A->nf, A->asc, A->aux);
     cuda_ok(cudaGetLastError(), "adj_dt_apply");
 }
 
@@ -437,7 +378,7 @@ void upload_seed(r3d_gpu* g, Adjoint* A, const double* const* seed) {
                     const int64_t ii = wrap(i, npx), jj = wrap(j, npy);
                     plane[(size_t)(k * g->geo.plane + jj * g->geo.pitch + ii)] += v;
                 }
-        cuda_ok(cudaMemcpyAsync(state_field(A->lam, A, f), plane.data(), plane.size() * sizeof(double),
+        cuda_ok(cudaMemcpyAsync(state_field(A->lam[A->cur], A, f), plane.data(), plane.size() * sizeof(double),
                                 cudaMemcpyHostToDevice, g->stream),
                 "seed upload");
         cuda_ok(cudaStreamSynchronize(g->stream), "seed upload");
@@ -449,7 +390,7 @@ void download_grad(r3d_gpu* g, Adjoint* A, double* const* grad) {
     std::vector<double> plane((size_t)g->geo.plane * NZ);
     for (int f = 0; f < A->nf; ++f) {
         if (!grad[f]) throw std::invalid_argument("null gradient field");
-        cuda_ok(cudaMemcpyAsync(plane.data(), state_field(A->lam, A, f), plane.size() * sizeof(double),
+        cuda_ok(cudaMemcpyAsync(plane.data(), state_field(A->lam[A->cur], A, f), plane.size() * sizeof(double),
                                 cudaMemcpyDeviceToHost, g->stream),
                 "gradient download");
         cuda_ok(cudaStreamSynchronize(g->stream), "gradient download");
@@ -483,9 +424,9 @@ void adjoint_free(r3d_gpu* g) {
     for (auto& s : A->S) cudaFree(s.base);
     cudaFree(A->Zb);
     for (double* p : A->F) cudaFree(p);
-    cudaFree(A->lam);
-    for (double* p : A->lamF) cudaFree(p);
-    cudaFree(A->Lam);
+    for (double* p : A->lam) cudaFree(p);
+    cudaFree(A->a);
+    cudaFree(A->mid);
     cudaFree(A->dots);
     cudaFree(A->asc);
     cudaFree(A->aux);

@@ -206,6 +206,42 @@ cudaError_t launch_dt_full(const Geometry& g, const Physics& ph, const Lines& L,
 }
 
 // ---------------------------------------------------------------------------------------
+// The lowest interior cell holding the limit that set dt (for the adjoint; the limits are
+// re-evaluated with the expressions that produced them, so the comparison is exact).
+// ---------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) dt_argmin_kernel(Geometry g, Physics ph, Lines L, FieldSet fs,
+                                                        const unsigned long long* key, unsigned long long* argmin) {
+    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = 1 + blockIdx.z;
+    if (i > g.npx || j > g.npy) return;
+    double mstar;
+    const int term = winning_limit(key, ph.lmag, mstar);
+    if (term == 3) return;  // the constant magnetic-diffusion limit has no derivative
+    const int n = k * (int)g.plane + j * (int)g.pitch + i;
+    double b2 = 0.0;
+    if (ph.lmag) {
+        const double bx = fs.xin[5][n], by = fs.xin[6][n], bz = fs.xin[7][n];
+        b2 = bx * bx + by * by + bz * bz;
+    }
+    const double dxy = (L.ddy[j] < L.ddx[i]) ? L.ddy[j] : L.ddx[i];
+    const double dd = (L.ddz[k] < dxy) ? L.ddz[k] : dxy;  // the dt_full_kernel expression
+    double w1, w2, w3, w4, um;
+    dt_terms(ph, fs.xin[0][n], fs.xin[1][n], fs.xin[2][n], fs.xin[3][n], fs.xin[4][n], b2, dd, L.rkapa[k], w1,
+             w2, w3, w4, um);
+    const double wq = term == 0 ? w1 : (term == 1 ? w2 : w3);
+    if (wq == mstar) atomicMin(argmin, (unsigned long long)n);
+}
+
+cudaError_t launch_dt_argmin(const Geometry& g, const Physics& ph, const Lines& L, const FieldSet& fs,
+                             const unsigned long long* key, unsigned long long* argmin, cudaStream_t st) {
+    dim3 block(32, 8, 1);
+    dim3 grid((g.npx + 31) / 32, (g.npy + 7) / 8, (unsigned)g.npz);
+    dt_argmin_kernel<<<grid, block, 0, st>>>(g, ph, L, fs, key, argmin);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------------------
 // Scalar bookkeeping: dt = sff*min(...) and umach = sqrt(max(...)) at the start of a step
 // (src/step.cpp:133-141, 224-229), and nit/timc/timt at its end (src/step.cpp:254-256).
 // ---------------------------------------------------------------------------------------

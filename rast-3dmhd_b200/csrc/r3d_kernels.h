@@ -76,6 +76,10 @@ cudaError_t launch_bcon(const Geometry& g, const Physics& ph, const Lines& L, co
 // only_refold: run only if step_end requested a re-evaluation (Scalars::refold)
 cudaError_t launch_dt_full(const Geometry& g, const Physics& ph, const Lines& L,
                            const FieldSet& fs, Scalars* sc, cudaStream_t st, int only_refold = 0);
+// the lowest cell whose limit equals the minimum that set dt (its keys: CFL, conduction, viscosity,
+// resistivity), into *argmin (set to ~0 before)
+cudaError_t launch_dt_argmin(const Geometry& g, const Physics& ph, const Lines& L, const FieldSet& fs,
+                             const unsigned long long* key, unsigned long long* argmin, cudaStream_t st);
 cudaError_t launch_step_begin(const Physics& ph, Scalars* sc, cudaStream_t st);
 // check: verify the filtered limits of a full step (Scalars::thr_*), request a refold if needed
 cudaError_t launch_step_end(Scalars* sc, cudaStream_t st, int check = 0);

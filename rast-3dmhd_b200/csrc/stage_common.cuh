@@ -103,6 +103,18 @@ __device__ __forceinline__ double min_of3(double a, double b, double c) {
 __device__ __forceinline__ double fold_min(double acc, double v) { return (v < acc) ? v : acc; }
 __device__ __forceinline__ double fold_max(double acc, double v) { return (acc < v) ? v : acc; }
 
+// The limit that sets dt, chosen from the four minima's keys as step_begin_kernel does: 0 CFL,
+// 1 conduction, 2 viscosity, 3 resistivity; m receives its value.
+__device__ __forceinline__ int winning_limit(const unsigned long long* key, int lmag, double& m) {
+    int t = 0;
+    m = order_value(key[0]);
+    const double w1 = order_value(key[1]), w2 = order_value(key[2]), w3 = order_value(key[3]);
+    if (w1 < m) { t = 1; m = w1; }
+    if (w2 < m) { t = 2; m = w2; }
+    if (lmag && w3 < m) { t = 3; m = w3; }
+    return t;
+}
+
 // Block-wide fold of the running limits, then one atomic per quantity into the scalars.
 // red must hold 5 doubles per warp.  Every thread of the block must call it.
 __device__ __forceinline__ void reduce_dt(double* red, double w1, double w2, double w3,
