@@ -3,9 +3,11 @@
 // The reference has no adjoint; this is the derivative of exactly the map the forward kernels
 // compute (src/step.cpp:114-257 with FLUXES, BCON and the dt reduction).  A trajectory of N
 // steps is recorded by the ordinary forward path, keeping the state every K steps on the
-// device.  The backward sweep walks the segments in reverse: it recomputes the states of a
-// segment from its checkpoint, then for each step (last first) recomputes the three stages
-// once more - now also storing the right-hand sides F_s (stage kernels with EMIT) - and runs
+// device and every step's limit minima (32 bytes).  The backward sweep walks the segments in
+// reverse: it recomputes the states of a segment from its checkpoint, each step's third stage
+// writing straight into the next state's buffer, then for each step (last first) recomputes the
+// three stages once more - now also storing the right-hand sides F_s (stage kernels with EMIT) -
+// and runs
 //
 //   for s = 2, 1, 0:   lambda_Y   = BCON^T lambda_X_{s+1}                       (adj_bcon_kernel)
 //                      lambda_F_s = gam_s dt lambda_Y + zeta_{s+1} dt lambda_Y(s+1)  (adj_pass1_kernel)
@@ -99,9 +101,18 @@ __global__ void __launch_bounds__(BX* BY, 2) adj_pass2_kernel(const __grid_const
     if (i <= A.g.npx && j <= A.g.npy) r3dk::adj_pass2_cell<MHD>(A, i, j, k);
 }
 
-__global__ void adj_save_limits_kernel(const r3dk::Scalars* sc, AdjScalars* aux) {
-    for (int q = 0; q < 4; ++q) aux->wkey[q] = sc->wmin[q];
+// Start of a recomputed step: its dt from the limit minima it started with (as step_begin_kernel
+// forms it), and thresholds under which the third stage evaluates no limits - the recompute
+// needs none.
+__global__ void adj_begin_kernel(r3dk::Physics ph, const unsigned long long* key, r3dk::Scalars* sc, AdjScalars* aux) {
+    for (int q = 0; q < 4; ++q) aux->wkey[q] = key[q];
     aux->argmin = ~0ull;
+    double m;
+    r3dk::winning_limit(aux->wkey, ph.lmag, m);
+    sc->dt = ph.sff * m;
+    sc->thr_on = 1;
+    sc->thr_w1 = 0.0;
+    sc->thr_um = 1e308;
 }
 
 // The n dot-product partials of the step's passes to kDotBlocks sums, each over a fixed share in
@@ -158,16 +169,11 @@ __global__ void __launch_bounds__(BX* BY) adj_compare_kernel(r3dk::Geometry g, c
 
 namespace r3dg {
 
-// A state: nf fields stored back to back, field f at base + f*field_elems (padded layout).
-struct StateBuf {
-    double* base = nullptr;
-    r3dk::StageMaps maps{};
-};
-
+// A state is nf fields stored back to back, field f at base + f*field_elems (padded layout).
 struct Adjoint {
     int nf = 5;
     int64_t field_elems = 0;
-    StateBuf S[4];                  // X_0 .. X_3 of the step being reversed
+    double* S[4] = {};              // X_1 .. X_3 of the step being recomputed; S[0]: the start state of adjoint_step
     double* Zb = nullptr;           // accumulator Z (nf fields)
     double* F[3] = {};              // F_0 .. F_2 (nf fields each)
     double* lam[2] = {};            // lambda_X / lambda_Y of a stage and of the one after it
@@ -181,7 +187,9 @@ struct Adjoint {
     AdjScalars* aux = nullptr;
     AdjScalars* haux = nullptr;     // pinned mirror
     std::vector<double*> ckpt;      // recorded checkpoints
-    std::vector<double*> seg;       // states of the segment being reversed
+    std::vector<double*> seg;       // states of the segment being reversed (its first is the checkpoint)
+    unsigned long long* lim = nullptr;  // recorded limit minima, four keys per step
+    int lim_steps = 0;
     int nsteps = 0, every = 0;
     bool recorded = false;
     int64_t bytes = 0;
@@ -217,15 +225,7 @@ Adjoint* workspace(r3d_gpu* g) {
         A->nf = g->nfields;
         A->field_elems = g->geo.plane * (g->geo.npz + 2);
         const size_t st = (size_t)A->nf * A->field_elems;
-        unsigned bx = 0, by = 0;
-        r3dk::stage_fp64_box(g->geo.tile_rows, &bx, &by);
-        for (int s = 0; s < 4; ++s) {
-            A->S[s].base = dalloc(A, st);
-            for (int f = 0; f < A->nf; ++f)
-                A->S[s].maps.m[f] = field_map(state_field(A->S[s].base, A, f), g->d.nx, g->d.ny, g->d.nz,
-                                              g->geo.pitch, g->geo.plane, bx, by,
-                                              CU_TENSOR_MAP_DATA_TYPE_FLOAT64, sizeof(double));
-        }
+        for (int s = 1; s < 4; ++s) A->S[s] = dalloc(A, st);
         A->Zb = dalloc(A, st);
         for (int s = 0; s < 3; ++s) A->F[s] = dalloc(A, st);
         for (int s = 0; s < 2; ++s) A->lam[s] = dalloc(A, st);
@@ -260,6 +260,19 @@ void free_states(std::vector<double*>& v) {
     v.clear();
 }
 
+// n state buffers, keeping those that are there (the excess is given back).
+void resize_states(const Adjoint* A, std::vector<double*>& v, int n) {
+    while ((int)v.size() > n) {
+        cudaFree(v.back());
+        v.pop_back();
+    }
+    while ((int)v.size() < n) {
+        double* p = nullptr;
+        cuda_ok(cudaMalloc(&p, (size_t)A->nf * A->field_elems * sizeof(double)), "cudaMalloc(states)");
+        v.push_back(p);
+    }
+}
+
 // Copy the simulation's current state (separate field arrays) into a contiguous state buffer.
 void save_current(r3d_gpu* g, Adjoint* A, double* dst) {
     const size_t nb = (size_t)A->field_elems * sizeof(double);
@@ -268,46 +281,56 @@ void save_current(r3d_gpu* g, Adjoint* A, double* dst) {
                 "checkpoint copy");
 }
 
-void copy_state(r3d_gpu* g, Adjoint* A, double* dst, const double* src) {
-    if (dst == src) return;
-    cuda_ok(cudaMemcpyAsync(dst, src, (size_t)A->nf * A->field_elems * sizeof(double), cudaMemcpyDeviceToDevice,
-                            g->stream),
-            "state copy");
+// The z ghost planes of a state buffer: constants that every stage reads and none writes.
+void copy_ghost_planes(r3d_gpu* g, Adjoint* A, double* dst, const double* src) {
+    const size_t pitch = (size_t)A->field_elems * sizeof(double), width = (size_t)g->geo.plane * sizeof(double);
+    for (int64_t k : {(int64_t)0, (int64_t)g->geo.npz + 1})
+        cuda_ok(cudaMemcpy2DAsync(dst + k * g->geo.plane, pitch, src + k * g->geo.plane, pitch, width, A->nf,
+                                  cudaMemcpyDeviceToDevice, g->stream),
+                "ghost planes");
 }
 
-r3dk::FieldSet stage_fields(const Adjoint* A, int s) {
+r3dk::FieldSet stage_fields(const Adjoint* A, int s, const double* in, double* out) {
     r3dk::FieldSet fs{};
     for (int f = 0; f < A->nf; ++f) {
-        fs.xin[f] = state_field(A->S[s].base, A, f);
-        fs.xout[f] = state_field(A->S[s + 1].base, A, f);
+        fs.xin[f] = in + (size_t)f * A->field_elems;
+        fs.xout[f] = out + (size_t)f * A->field_elems;
         fs.z[f] = state_field(A->Zb, A, f);
         fs.f[f] = state_field(A->F[s], A, f);
     }
     return fs;
 }
 
-// One forward step from S[0] (a copy of src) with every intermediate kept: S[1..3], F[0..2],
-// and the limits/dt of the step in asc/aux.
-void recompute_step(r3d_gpu* g, Adjoint* A, const double* src) {
-    copy_state(g, A, A->S[0].base, src);
-    cuda_ok(r3dk::launch_reset_reduction(A->asc, g->stream), "adjoint reset");
-    r3dk::FieldSet f0 = stage_fields(A, 0);
-    cuda_ok(r3dk::launch_dt_full(g->geo, g->ph, g->lines, f0, A->asc, g->stream), "adjoint dt_full");
-    adj_save_limits_kernel<<<1, 1, 0, g->stream>>>(A->asc, A->aux);
-    cuda_ok(cudaGetLastError(), "adjoint save limits");
-    cuda_ok(r3dk::launch_step_begin(g->ph, A->asc, g->stream), "adjoint step_begin");
+r3dk::StageMaps state_maps(const r3d_gpu* g, const Adjoint* A, const double* base) {
+    r3dk::StageMaps m{};
+    unsigned bx = 0, by = 0;
+    r3dk::stage_fp64_box(g->geo.tile_rows, &bx, &by);
+    for (int f = 0; f < A->nf; ++f)
+        m.m[f] = field_map(const_cast<double*>(base) + (size_t)f * A->field_elems, g->d.nx, g->d.ny, g->d.nz,
+                           g->geo.pitch, g->geo.plane, bx, by, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, sizeof(double));
+    return m;
+}
+
+// One forward step from the state src with the dt of the limit minima key, through S[1] and S[2]
+// into dst; emit: F[0..2] stored.
+void recompute_step(r3d_gpu* g, Adjoint* A, const unsigned long long* key, const double* src, double* dst, bool emit) {
+    adj_begin_kernel<<<1, 1, 0, g->stream>>>(g->ph, key, A->asc, A->aux);
+    cuda_ok(cudaGetLastError(), "adjoint begin");
+    const double* in[3] = {src, A->S[1], A->S[2]};
+    double* out[3] = {A->S[1], A->S[2], dst};
     for (int s = 0; s < 3; ++s) {
-        r3dk::FieldSet fs = stage_fields(A, s);
-        cuda_ok(r3dk::launch_stage_fp64(s, A->S[s].maps, g->geo, g->ph, g->lines, fs, A->asc, g->kchunk, g->stream,
-                                        true),
+        r3dk::FieldSet fs = stage_fields(A, s, in[s], out[s]);
+        cuda_ok(r3dk::launch_stage_fp64(s, state_maps(g, A, in[s]), g->geo, g->ph, g->lines, fs, A->asc, g->kchunk,
+                                        g->stream, emit),
                 "adjoint recompute stage");
         cuda_ok(r3dk::launch_bcon(g->geo, g->ph, g->lines, g->bnd, fs, A->asc, 0, g->stream), "adjoint bcon");
     }
 }
 
-// Reverse the step whose intermediates recompute_step left in the workspace: lam[cur] holds the
-// adjoint of X_3 on entry and of X_0 on exit.
-void reverse_step(r3d_gpu* g, Adjoint* A) {
+// Reverse the step from src whose intermediates recompute_step left in S[1..3] and F: lam[cur]
+// holds the adjoint of X_3 on entry and of X_0 = src on exit.
+void reverse_step(r3d_gpu* g, Adjoint* A, const double* src) {
+    const double* X[4] = {src, A->S[1], A->S[2], A->S[3]};
     const dim3 blk(BX, BY, 1), cg = cell_grid(g);
     const dim3 cols(cg.x, cg.y, g->geo.npz < 6 ? 1 : 2);
     const bool mhd = A->nf == 8;
@@ -316,7 +339,7 @@ void reverse_step(r3d_gpu* g, Adjoint* A) {
         double* other = A->lam[1 - A->cur];  // lambda_Y of stage s + 1, then lambda_X of stage s
         FieldPtrs fp{};
         for (int f = 0; f < A->nf; ++f) {
-            fp.x[f] = state_field(A->S[s + 1].base, A, f);
+            fp.x[f] = X[s + 1] + (size_t)f * A->field_elems;
             fp.lam[f] = state_field(lam, A, f);
         }
         adj_bcon_kernel<<<cols, blk, 0, g->stream>>>(g->geo, g->ph, g->bnd, fp, A->nf);
@@ -326,7 +349,7 @@ void reverse_step(r3d_gpu* g, Adjoint* A) {
         p.ph = g->ph;
         p.L = g->lines;
         p.fe = A->field_elems;
-        p.x = A->S[s].base;
+        p.x = X[s];
         p.lam = lam;
         p.lprev = s < 2 ? other : nullptr;
         p.a = A->a;
@@ -347,10 +370,11 @@ void reverse_step(r3d_gpu* g, Adjoint* A) {
     }
     adj_dots_kernel<<<kDotBlocks, kSumThreads, 0, g->stream>>>(A->dots, 3 * A->nblocks, A->aux);
     cuda_ok(cudaGetLastError(), "adj_dots");
-    cuda_ok(r3dk::launch_dt_argmin(g->geo, g->ph, g->lines, stage_fields(A, 0), A->aux->wkey, &A->aux->argmin, g->stream),
+    cuda_ok(r3dk::launch_dt_argmin(g->geo, g->ph, g->lines, stage_fields(A, 0, src, A->S[1]), A->aux->wkey,
+                                   &A->aux->argmin, g->stream),
             "adj_argmin");
-    adj_dt_apply_kernel<<<1, 1, 0, g->stream>>>(g->geo, g->ph, g->lines, A->S[0].base, A->lam[A->cur], A->field_elems,
-                                               A->nf, A->asc, A->aux);
+    adj_dt_apply_kernel<<<1, 1, 0, g->stream>>>(g->geo, g->ph, g->lines, src, A->lam[A->cur], A->field_elems, A->nf,
+                                                A->asc, A->aux);
     cuda_ok(cudaGetLastError(), "adj_dt_apply");
 }
 
@@ -421,7 +445,8 @@ void check_aux(r3d_gpu* g, Adjoint* A) {
 void adjoint_free(r3d_gpu* g) {
     Adjoint* A = g->adj;
     if (!A) return;
-    for (auto& s : A->S) cudaFree(s.base);
+    for (double* p : A->S) cudaFree(p);
+    cudaFree(A->lim);
     cudaFree(A->Zb);
     for (double* p : A->F) cudaFree(p);
     for (double* p : A->lam) cudaFree(p);
@@ -453,19 +478,23 @@ int r3d_gpu_adjoint_record(r3d_gpu* g, int nsteps, int checkpoint_every, r3d_sca
         Range r("r3d.adjoint_record");
         Adjoint* A = workspace(g);
         A->recorded = false;
-        free_states(A->ckpt);
         // checkpoints at steps 0, K, 2K, .. and the final state (compared against in backward)
         const int nck = (nsteps + checkpoint_every - 1) / checkpoint_every + 1;
-        const size_t st = (size_t)A->nf * A->field_elems;
-        for (int c = 0; c < nck; ++c) {
-            double* p = nullptr;
-            cuda_ok(cudaMalloc(&p, st * sizeof(double)), "cudaMalloc(checkpoint)");
-            A->ckpt.push_back(p);
+        resize_states(A, A->ckpt, nck);
+        if (nsteps > A->lim_steps) {
+            cudaFree(A->lim);
+            A->lim = nullptr;
+            A->lim_steps = 0;
+            cuda_ok(cudaMalloc(&A->lim, (size_t)nsteps * sizeof(g->dsc->wmin)), "cudaMalloc(limits)");
+            A->lim_steps = nsteps;
         }
         Timer tm{g, false, nullptr};
         int launches = 0, stage_launches = 0;
         for (int n = 0; n < nsteps; ++n) {
             if (n % checkpoint_every == 0) save_current(g, A, A->ckpt[n / checkpoint_every]);
+            cuda_ok(cudaMemcpyAsync(A->lim + 4 * n, g->dsc->wmin, sizeof(g->dsc->wmin), cudaMemcpyDeviceToDevice,
+                                    g->stream),
+                    "record limits");
             enqueue_step(g, 3, tm, launches, stage_launches);
         }
         save_current(g, A, A->ckpt.back());
@@ -483,32 +512,26 @@ int r3d_gpu_adjoint_backward(r3d_gpu* g, const double* const* seed, double* cons
         DeviceGuard dg(g->device);
         Range r("r3d.adjoint_backward");
         Adjoint* A = g->adj;
-        const size_t st = (size_t)A->nf * A->field_elems;
-        // the recompute buffers start as copies of X_0: their z ghost planes are constants
-        for (int s = 1; s < 4; ++s) copy_state(g, A, A->S[s].base, A->ckpt[0]);
+        const int K = A->every, N = A->nsteps;
+        // states 1 .. K-1 of a segment; the recompute buffers take the constant z ghost planes of X_0
+        resize_states(A, A->seg, std::min(K, N) - 1);
+        for (int s = 1; s < 4; ++s) copy_ghost_planes(g, A, A->S[s], A->ckpt[0]);
+        for (double* p : A->seg) copy_ghost_planes(g, A, p, A->ckpt[0]);
         cuda_ok(cudaMemsetAsync(&A->aux->mismatch, 0, sizeof(unsigned long long), g->stream), "cudaMemset");
         upload_seed(g, A, seed);
-        const int K = A->every, N = A->nsteps;
-        while ((int)A->seg.size() < K) {
-            double* p = nullptr;
-            cuda_ok(cudaMalloc(&p, st * sizeof(double)), "cudaMalloc(segment)");
-            A->seg.push_back(p);
-        }
         const double* final_state = A->ckpt.back();  // the recorded final state
         {
             const int nseg = (N + K - 1) / K;
             for (int sg = nseg - 1; sg >= 0; --sg) {
                 const int s0 = sg * K, len = std::min(K, N - s0);
-                copy_state(g, A, A->seg[0], A->ckpt[sg]);
-                for (int s = 1; s < len; ++s) {
-                    recompute_step(g, A, A->seg[s - 1]);
-                    copy_state(g, A, A->seg[s], A->S[3].base);
-                }
+                auto state = [&](int s) -> double* { return s == 0 ? A->ckpt[sg] : A->seg[s - 1]; };
+                for (int s = 1; s < len; ++s)
+                    recompute_step(g, A, A->lim + 4 * (s0 + s - 1), state(s - 1), state(s), false);
                 for (int s = len - 1; s >= 0; --s) {
-                    recompute_step(g, A, A->seg[s]);
-                    const double* next = s + 1 < len ? A->seg[s + 1] : (sg + 1 < nseg ? A->ckpt[sg + 1] : final_state);
-                    compare_states(g, A, A->S[3].base, next);
-                    reverse_step(g, A);
+                    recompute_step(g, A, A->lim + 4 * (s0 + s), state(s), A->S[3], true);
+                    const double* next = s + 1 < len ? state(s + 1) : (sg + 1 < nseg ? A->ckpt[sg + 1] : final_state);
+                    compare_states(g, A, A->S[3], next);
+                    reverse_step(g, A, state(s));
                 }
                 check_aux(g, A);
             }
@@ -523,11 +546,15 @@ int r3d_gpu_adjoint_step(r3d_gpu* g, const double* const* seed, double* const* g
         if (!g->uploaded) throw Error(R3D_ESTATE, "adjoint before upload");
         DeviceGuard dg(g->device);
         Adjoint* A = workspace(g);
-        save_current(g, A, A->S[0].base);
-        for (int s = 1; s < 4; ++s) copy_state(g, A, A->S[s].base, A->S[0].base);
+        if (!A->S[0]) A->S[0] = dalloc(A, (size_t)A->nf * A->field_elems);
+        save_current(g, A, A->S[0]);
+        for (int s = 1; s < 4; ++s) copy_ghost_planes(g, A, A->S[s], A->S[0]);
         upload_seed(g, A, seed);
-        recompute_step(g, A, A->S[0].base);
-        reverse_step(g, A);
+        cuda_ok(r3dk::launch_reset_reduction(A->asc, g->stream), "adjoint reset");
+        cuda_ok(r3dk::launch_dt_full(g->geo, g->ph, g->lines, stage_fields(A, 0, A->S[0], A->S[1]), A->asc, g->stream),
+                "adjoint dt_full");
+        recompute_step(g, A, A->asc->wmin, A->S[0], A->S[3], true);
+        reverse_step(g, A, A->S[0]);
         check_aux(g, A);
         download_grad(g, A, grad);
     });

@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
                     if (gdx && gdy) fs.xout[f][nc + gdx + gdy] = xn[f];
                 }
             }
-            if (STAGE == 2 && !edge) {
+            if (STAGE == 2 && !EMIT && !edge) {  // the adjoint's recompute needs no limits
                 const double dd = (L.ddz[k] < dxyv[c]) ? L.ddz[k] : dxyv[c];  // min_of3(ddx, ddy, ddz)
                 double b2sum = 0.0;
                 if constexpr (MHD) b2sum = xn[5] * xn[5] + xn[6] * xn[6] + xn[7] * xn[7];
@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
         }
         return;
     }
-    if (STAGE == 2) reduce_dt(der, m1, m2, m3, m4, mu, sc);
+    if (STAGE == 2 && !EMIT) reduce_dt(der, m1, m2, m3, m4, mu, sc);
 }
 
 template <int STAGE, bool KC, bool MHD, bool EMIT, int TYV, bool TF, bool IDD>
