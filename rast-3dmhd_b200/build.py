@@ -16,7 +16,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off,-O2",
           "-I", os.path.join(ROOT, "include"), "-I", os.path.join(PKG, "host"), "-I", os.path.join(PKG, "csrc")]
-HOST_SRCS = ["host/params.cpp", "host/setup.cpp"]
+HOST_SRCS = ["host/params.cpp", "host/setup.cpp", "host/hostcopy.cpp"]
 # FMA contraction: off everywhere the FP64 result must equal the reference CPU build; on for
 # the FP32-bulk kernels and the reverse sweep, which carry no bit-exactness contract (the search
 # for the cell that set dt compares exactly and is compiled with bcon.cu).
@@ -56,7 +56,7 @@ def build(verbose_ptxas: bool = False, force: bool = False) -> str:
             extra = ["-Xptxas", "-v"] if (verbose_ptxas and s.endswith(".cu")) else []
             lang = ["-x", "cu"] if s.endswith(".cu") else ["-x", "c++"]
             fmad = ["-fmad=true"] if s in FMAD_ON else ["-fmad=false"]
-            omp = ["-Xcompiler", "-fopenmp"] if s in HOST_SRCS else []  # host set-up loops
+            omp = ["-Xcompiler", "-fopenmp"] if s in HOST_SRCS else []  # host set-up loops and copies
             _run([NVCC] + ARCH + COMMON + fmad + omp + extra + lang + ["-c", src, "-o", obj])
     if force or _stale(LIB, objs):
         _run([NVCC] + ARCH + ["-shared", "-Xcompiler", "-fPIC", "-o", LIB] + objs +

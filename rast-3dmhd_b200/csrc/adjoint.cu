@@ -101,6 +101,25 @@ __global__ void __launch_bounds__(BX* BY, 2) adj_pass2_kernel(const __grid_const
     if (i <= A.g.npx && j <= A.g.npy) r3dk::adj_pass2_cell<MHD>(A, i, j, k);
 }
 
+// Interior cells of lam from a cotangent in the reference layout: the cell's own entry and those of
+// its periodic ghost images, added in (j, i) order.
+__global__ void __launch_bounds__(BX* BY) adj_seed_fold_kernel(r3dk::Geometry g, const double* seed, double* lam) {
+    const int i = 1 + blockIdx.x * BX + threadIdx.x;
+    const int j = 1 + blockIdx.y * BY + threadIdx.y;
+    const int k = 1 + blockIdx.z;
+    if (i > g.npx || j > g.npy) return;
+    const int64_t nx = g.npx + 2, ny = g.npy + 2;
+    auto row = [&](int64_t jj) {  // entries at i = 0 (the image of npx), i, npx + 1 (of 1)
+        const double* s = seed + (k * ny + jj) * nx;
+        double v = i == g.npx ? s[0] + s[i] : s[i];
+        if (i == 1) v += s[g.npx + 1];
+        return v;
+    };
+    double v = j == g.npy ? row(0) + row(j) : row(j);
+    if (j == 1) v += row(g.npy + 1);
+    lam[(int64_t)k * g.plane + (int64_t)j * g.pitch + i] = v;
+}
+
 // Start of a recomputed step: its dt from the limit minima it started with (as step_begin_kernel
 // forms it), and thresholds under which the third stage evaluates no limits - the recompute
 // needs none.
@@ -385,47 +404,31 @@ void compare_states(r3d_gpu* g, Adjoint* A, const double* a, const double* b) {
 }
 
 // Host cotangent (NX*NY*NZ per field, ghosts included) -> lam: x/y ghost entries are added to
-// the interior cells they image, z ghost planes are constants and dropped.
+// the interior cells they image, z ghost planes are constants and dropped.  The fields pass through
+// F[0], which holds nothing between steps.  (Folding on the host, cell by cell, and copying the
+// gradient back the same way took 60 of the 64 ms of a 128x128x128 hydro adjoint_step.)
 void upload_seed(r3d_gpu* g, Adjoint* A, const double* const* seed) {
-    const int64_t NX = g->d.nx, NY = g->d.ny, NZ = g->d.nz;
-    const int npx = g->p.npx, npy = g->p.npy;
-    std::vector<double> plane((size_t)g->geo.plane * NZ);
-    auto wrap = [](int64_t q, int64_t np) { return q == 0 ? np : (q == np + 1 ? 1 : q); };
-    for (int f = 0; f < A->nf; ++f) {
+    for (int f = 0; f < A->nf; ++f)
         if (!seed[f]) throw std::invalid_argument("null seed field");
-        std::fill(plane.begin(), plane.end(), 0.0);
-        for (int64_t k = 1; k <= NZ - 2; ++k)
-            for (int64_t j = 0; j < NY; ++j)
-                for (int64_t i = 0; i < NX; ++i) {
-                    const double v = seed[f][(k * NY + j) * NX + i];
-                    if (v == 0.0) continue;
-                    const int64_t ii = wrap(i, npx), jj = wrap(j, npy);
-                    plane[(size_t)(k * g->geo.plane + jj * g->geo.pitch + ii)] += v;
-                }
-        cuda_ok(cudaMemcpyAsync(state_field(A->lam[A->cur], A, f), plane.data(), plane.size() * sizeof(double),
-                                cudaMemcpyHostToDevice, g->stream),
-                "seed upload");
-        cuda_ok(cudaStreamSynchronize(g->stream), "seed upload");
+    const int64_t NX = g->d.nx, NY = g->d.ny, NZ = g->d.nz;
+    const dim3 blk(BX, BY, 1), gr = cell_grid(g);
+    for (int f = 0; f < A->nf; ++f) {
+        double* stage = state_field(A->F[0], A, f);
+        from_host(g, stage, seed[f], (size_t)(NX * NY * NZ) * sizeof(double), "seed upload");
+        adj_seed_fold_kernel<<<gr, blk, 0, g->stream>>>(g->geo, stage, state_field(A->lam[A->cur], A, f));
+        cuda_ok(cudaGetLastError(), "adj_seed_fold");
     }
+    cuda_ok(cudaStreamSynchronize(g->stream), "seed upload");  // the caller's arrays are free again
 }
 
 void download_grad(r3d_gpu* g, Adjoint* A, double* const* grad) {
-    const int64_t NX = g->d.nx, NY = g->d.ny, NZ = g->d.nz;
-    std::vector<double> plane((size_t)g->geo.plane * NZ);
-    for (int f = 0; f < A->nf; ++f) {
+    for (int f = 0; f < A->nf; ++f)
         if (!grad[f]) throw std::invalid_argument("null gradient field");
-        cuda_ok(cudaMemcpyAsync(plane.data(), state_field(A->lam[A->cur], A, f), plane.size() * sizeof(double),
-                                cudaMemcpyDeviceToHost, g->stream),
-                "gradient download");
-        cuda_ok(cudaStreamSynchronize(g->stream), "gradient download");
-        for (int64_t k = 0; k < NZ; ++k)
-            for (int64_t j = 0; j < NY; ++j)
-                for (int64_t i = 0; i < NX; ++i) {
-                    const bool inner = k >= 1 && k <= NZ - 2 && j >= 1 && j <= NY - 2 && i >= 1 && i <= NX - 2;
-                    grad[f][(k * NY + j) * NX + i] =
-                        inner ? plane[(size_t)(k * g->geo.plane + j * g->geo.pitch + i)] : 0.0;
-                }
-    }
+    // lam's ghost cells are zero: nothing writes them
+    for (int f = 0; f < A->nf; ++f)
+        to_host(g, grad[f], state_field(A->lam[A->cur], A, f), g->geo.pitch * sizeof(double), g->d.nx * sizeof(double),
+                g->d.ny * g->d.nz, "gradient download");
+    cuda_ok(cudaStreamSynchronize(g->stream), "gradient download");
 }
 
 void check_aux(r3d_gpu* g, Adjoint* A) {

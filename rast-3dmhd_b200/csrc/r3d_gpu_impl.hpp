@@ -66,6 +66,8 @@ struct r3d_gpu {
     // replays it; six stages leave the parity unchanged)
     cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
     int64_t steps_enqueued = 0;
+    void* bounce[2] = {nullptr, nullptr};  // page-locked copy buffers (to_host, from_host)
+    cudaEvent_t bounce_ev[2] = {nullptr, nullptr};
 };
 
 namespace r3dg {
@@ -139,6 +141,12 @@ void destroy_handle(r3d_gpu* g);
 void enqueue_step_begin(r3d_gpu* g);
 void enqueue_stage(r3d_gpu* g, int s);  // stage s + BCON; the new state becomes current
 void enqueue_step_end(r3d_gpu* g, int nstages);
+// Copies between the device and the caller's arrays, rows of `width` bytes, dense on the host and
+// `pitch` bytes apart on the device, ordered on the handle's stream.  Page-locked host arrays are
+// copied directly (asynchronously); pageable ones through two page-locked buffers that the handle
+// keeps, the host side by several threads (done when the call returns).
+void to_host(r3d_gpu* g, void* dst, const void* src, size_t pitch, size_t width, size_t rows, const char* what);
+void from_host(r3d_gpu* g, void* dst, const void* src, size_t bytes, const char* what);
 // Device pointer and element size of field q of the current state (FP64 or FP32-bulk).
 void* state_field(r3d_gpu* g, int q, size_t* esize);
 int state_fields(const r3d_gpu* g);

@@ -97,4 +97,7 @@ void setup_state(const r3d_params& p, const r3d_host_state& st, r3d_scalars& sc,
 // domain: y rows first, then x columns).
 void fill_ghosts(double* f, int64_t nx, int64_t ny, int64_t nz);
 
+// memcpy by up to eight threads (hostcopy.cpp).
+void parallel_copy(void* dst, const void* src, size_t bytes);
+
 }  // namespace r3db
