@@ -204,7 +204,8 @@ int r3d_gpu_debug_dt_filter(r3d_gpu* g, double margin, int* refolds);
  * fill the GPU once takes the depth (down to 4) minimising waves x planes per chunk; a hydro
  * launch of up to 64 waves takes a slightly shallower depth (at most one chunk more) when a
  * list-scheduling estimate of the launch, whose last chunk's CTAs run last, finds it 0.5%
- * shorter. */
+ * shorter.  A handle cuts the planned chunks of a hydro launch of a few waves, or of less than one,
+ * finer still (R3D_KCHUNK is taken as it is). */
 int r3d_gpu_plan(const r3d_params* p, int nloc, int num_sms, int* kchunk, int* tile_rows);
 
 /* Bytes of device memory held by g. */

@@ -241,6 +241,42 @@ int plan_chunk_depth(int64_t tiles, int nloc, int d, int64_t slots) {
     return d;
 }
 
+// Planes per CTA of a hydro launch (FP64 or FP32-bulk): the planned depth, or a shallower cut of it
+// where the plan leaves SMs idle - launches of a few waves, whose last wave is partly empty, and
+// those of less than one.  The score is the mean of the list-scheduled length of the launch and of
+// its evenly spread work (a lone CTA runs about twice as fast as one that shares its SM, so a
+// partial wave costs about half of what list scheduling says), each CTA costing its planes plus
+// 0.3 for its start, and 15% over the number of waves more (CTAs that start together load and
+// compute in step); cuts into more than 8 waves are not considered, and the plan stays unless the
+// score improves by 2%.  B200, stage kernels of a step (planned depth: us; chosen depth: us):
+// 32x32x64 4: 59, 1: 38; 128x128x256 29: 639, 13: 551 (best, 10: 545); 400x100x50 12: 314, 5: 302;
+// FP32-bulk 126x126x256 32: 408, 7: 347 (6 and 8: 346, 347).  MHD keeps its plan (12- and 16-plane chunks measured
+// best or within 2% on 64x64x128, 80x330x61, 126x126x256 and 252x252x256).
+int launch_depth(int64_t tiles, int nloc, int planned, int64_t slots) {
+    constexpr double kStart = 0.3;
+    auto ctas = [&](int k) { return tiles * ((nloc + k - 1) / k); };
+    auto score = [&](int k) {
+        const int64_t full = tiles * (nloc / k), q = full / slots, r = full % slots;
+        const double w = k + kStart;
+        const int rem = nloc % k;
+        double end = (q + (r ? 1 : 0)) * w, work = full * w;
+        if (rem) {  // the last chunk's CTAs start on the slots that the partial wave leaves free
+            const double v = rem + kStart;
+            end = std::max(end, q * w + v * ((tiles + slots - r - 1) / (slots - r)));
+            work += tiles * v;
+        }
+        return (0.5 * end + 0.5 * work / slots) * (1.0 + 0.15 * slots / ctas(k));
+    };
+    int best = planned;
+    double low = score(planned) * 0.98;
+    for (int k = planned - 1; k >= 1 && ctas(k) <= 8 * slots; --k)
+        if (score(k) < low) {
+            best = k;
+            low = score(k);
+        }
+    return best;
+}
+
 // z-chunk depth (planes per CTA) of the stage kernels of a handle over nloc local planes, given
 // its precision, FP64 column-tile rows and the device's SM count; R3D_KCHUNK=<planes> in the
 // environment overrides it.
@@ -475,14 +511,14 @@ void enqueue_stage(r3d_gpu* g, int s) {
     if (g->fp32) {
         r3dk::FieldSet32 fs = fieldset32(g);
         cuda_ok(r3dk::launch_stage_fp32(s, g->maps[g->cur], g->geo, g->ph, g->lines, g->bg, fs, g->dsc,
-                                        g->kchunk, g->stream),
+                                        g->depth, g->stream),
                 "stage32");
         cuda_ok(r3dk::launch_bcon_fp32(g->geo, g->ph, g->lines, g->bnd, g->bg, fs, g->dsc, s == 2 ? 1 : 0, g->stream),
                 "bcon32");
     } else {
         FieldSet fs = fieldset(g);
         if (g->ph.id_mode) launch_plane_mean(g, fs);
-        cuda_ok(r3dk::launch_stage_fp64(s, g->maps[g->cur], g->geo, g->ph, g->lines, fs, g->dsc, g->kchunk, g->stream),
+        cuda_ok(r3dk::launch_stage_fp64(s, g->maps[g->cur], g->geo, g->ph, g->lines, fs, g->dsc, g->depth, g->stream),
                 "stage");
         cuda_ok(r3dk::launch_bcon(g->geo, g->ph, g->lines, g->bnd, fs, g->dsc, s == 2 ? 1 : 0, g->stream), "bcon");
     }
@@ -512,7 +548,7 @@ void enqueue_step(r3d_gpu* g, int nstages, Timer& tm, int& launches, int& stage_
         tm.begin();
         if (g->fp32) {
             r3dk::FieldSet32 fs = fieldset32(g);
-            cuda_ok(r3dk::launch_stage_fp32(s, g->maps[g->cur], g->geo, g->ph, g->lines, g->bg, fs, g->dsc, g->kchunk, g->stream), "stage32");
+            cuda_ok(r3dk::launch_stage_fp32(s, g->maps[g->cur], g->geo, g->ph, g->lines, g->bg, fs, g->dsc, g->depth, g->stream), "stage32");
             tm.end(0);
             tm.begin();
             cuda_ok(r3dk::launch_bcon_fp32(g->geo, g->ph, g->lines, g->bnd, g->bg, fs, g->dsc, s == 2 ? 1 : 0, g->stream), "bcon32");
@@ -524,7 +560,7 @@ void enqueue_step(r3d_gpu* g, int nstages, Timer& tm, int& launches, int& stage_
                 ++launches;
                 tm.begin();
             }
-            cuda_ok(r3dk::launch_stage_fp64(s, g->maps[g->cur], g->geo, g->ph, g->lines, fs, g->dsc, g->kchunk, g->stream), "stage");
+            cuda_ok(r3dk::launch_stage_fp64(s, g->maps[g->cur], g->geo, g->ph, g->lines, fs, g->dsc, g->depth, g->stream), "stage");
             tm.end(0);
             tm.begin();
             cuda_ok(r3dk::launch_bcon(g->geo, g->ph, g->lines, g->bnd, fs, g->dsc, s == 2 ? 1 : 0, g->stream), "bcon");
@@ -955,6 +991,16 @@ r3d_gpu* create_handle(const r3d_params& pin, int z0, int nloc, cudaStream_t sha
             b.hh = p->hh; b.theta = p->theta; b.tp = p->tp; b.tpr = p->tp;
             b.half_nx = (int)(d.nx / 2);
             g->kchunk = stage_chunk_depth(*p, g->fp32, g->geo.tile_rows, nloc, g->num_sms);
+            {
+                unsigned tx = 0, ty = 0;
+                if (g->fp32) r3dk::stage_fp32_box(&tx, &ty);
+                else r3dk::stage_fp64_box(g->geo.tile_rows, &tx, &ty);
+                const int rows = (int)ty - 2;
+                const int64_t tiles = (int64_t)((p->npx + 31) / 32) * ((p->npy + rows - 1) / rows);
+                const int64_t slots = (int64_t)g->num_sms * (g->fp32 ? r3dk::stage_fp32_ctas_per_sm()
+                                                                     : r3dk::stage_fp64_ctas_per_sm(p->lmag, rows));
+                g->depth = (p->lmag || getenv("R3D_KCHUNK")) ? g->kchunk : launch_depth(tiles, nloc, g->kchunk, slots);
+            }
             cuda_ok(cudaStreamSynchronize(g->stream), "create");
     } catch (...) {
         destroy_handle(g);
@@ -1291,7 +1337,7 @@ void eval_fluxes(r3d_gpu* g, int buf, double* const* out) {
         fs.z[q] = g->fscr + (size_t)(nf + q) * fe;             // accumulator, discarded
         fs.f[q] = g->fscr + (size_t)(2 * nf + q) * fe;         // F
     }
-    cuda_ok(r3dk::launch_stage_fp64(0, g->maps[buf], g->geo, g->ph, g->lines, fs, g->dsc, g->kchunk, g->stream,
+    cuda_ok(r3dk::launch_stage_fp64(0, g->maps[buf], g->geo, g->ph, g->lines, fs, g->dsc, g->depth, g->stream,
                                     true),
             "fluxes");
     for (int q = 0; q < nf; ++q) {

@@ -46,7 +46,8 @@ struct r3d_gpu {
     r3dk::Scalars* dsc = nullptr;
     r3dk::Scalars* hsc = nullptr;  // pinned mirror
     int cur = 0;
-    int kchunk = 32;
+    int kchunk = 32;  // planned z-chunk depth (r3d_gpu_plan)
+    int depth = 32;   // planes per CTA of its stage launches (launch_depth)
     bool uploaded = false;
     bool work_ok = false;  // the last operation on the state was a full step (r3d_gpu_download_work)
     int64_t bytes = 0;
