@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(BX* BY) adj_seed_fold_kernel(r3dk::Geometry g,
 }
 
 // Start of a recomputed step: its dt from the limit minima it started with (as step_begin_kernel
-// forms it), and thresholds under which the third stage evaluates no limits - the recompute
+// forms it), and bounds under which the third stage skips every cell's limits - the recompute
 // needs none.
 __global__ void adj_begin_kernel(r3dk::Physics ph, const unsigned long long* key, r3dk::Scalars* sc, AdjScalars* aux) {
     for (int q = 0; q < 4; ++q) aux->wkey[q] = key[q];
@@ -129,9 +129,8 @@ __global__ void adj_begin_kernel(r3dk::Physics ph, const unsigned long long* key
     double m;
     r3dk::winning_limit(aux->wkey, ph.lmag, m);
     sc->dt = ph.sff * m;
-    sc->thr_on = 1;
-    sc->thr_w1 = 0.0;
-    sc->thr_um = 1e308;
+    sc->bnd = r3dk::DtBounds{};
+    sc->bnd.u = __int_as_float(0x7f800000);
 }
 
 // The n dot-product partials of the step's passes to kDotBlocks sums, each over a fixed share in

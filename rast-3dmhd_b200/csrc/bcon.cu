@@ -246,44 +246,11 @@ cudaError_t launch_dt_argmin(const Geometry& g, const Physics& ph, const Lines& 
 // (src/step.cpp:133-141, 224-229), and nit/timc/timt at its end (src/step.cpp:254-256).
 // ---------------------------------------------------------------------------------------
 __global__ void step_begin_kernel(Physics ph, Scalars* sc) {
-    const double w0 = order_value(sc->wmin[0]), w1 = order_value(sc->wmin[1]);
-    const double w2 = order_value(sc->wmin[2]), w3 = order_value(sc->wmin[3]);
-    double m = (w1 < w0) ? w1 : w0;
-    m = (w2 < m) ? w2 : m;
-    if (ph.lmag) m = (w3 < m) ? w3 : m;
-    sc->dt = ph.sff * m;
-    const double u = order_value(sc->umax);
-    sc->umach = sqrt(u);
-    // thresholds of this step's filtered fold: the previous limits widened by the margin (a
-    // margin < 0 forces the re-evaluation path; thr_on == 0 leaves only the exact running bounds);
-    // a slab takes its own limits, so that its check at step_end makes its own fold exact
-    const double tw = sc->thr_local ? order_value(sc->wloc[0]) : w0;
-    const double tu = sc->thr_local ? order_value(sc->uloc) : u;
-    sc->thr_w1 = sc->thr_on ? tw * (1.0 + sc->thr_margin) : 1e308;
-    sc->thr_um = sc->thr_on ? tu * (1.0 - sc->thr_margin) : 0.0;
-    sc->wmin[0] = sc->wmin[1] = sc->wmin[2] = sc->wmin[3] = order_key(1e300);
-    sc->umax = order_key(0.0);
+    step_begin(ph, sc);
+    clear_limits(sc);
 }
 
-// check != 0 (after a full step on a handle with the threshold filter): the skipped cells have
-// ww1 > thr_w1 and a Mach term < thr_um, so the folded limits are exact iff the minimum found
-// is <= thr_w1 and the maximum >= thr_um; otherwise clear them and request the full evaluation
-// (dt_full_kernel with only_refold).
-__global__ void step_end_kernel(Scalars* sc, int check) {
-    sc->nit += 1;
-    sc->timc += sc->dt;
-    sc->timt = sc->timi + sc->timc;
-    int refold = 0;
-    if (check && sc->thr_on) {
-        refold = !(order_value(sc->wmin[0]) <= sc->thr_w1) || !(order_value(sc->umax) >= sc->thr_um);
-        if (refold) {
-            sc->refolds += 1;
-            sc->wmin[0] = sc->wmin[1] = sc->wmin[2] = sc->wmin[3] = order_key(1e300);
-            sc->umax = order_key(0.0);
-        }
-    }
-    sc->refold = refold;
-}
+__global__ void step_end_kernel(Scalars* sc, int check) { step_end(sc, check); }
 
 __global__ void save_local_limits_kernel(Scalars* sc) {
     for (int q = 0; q < 4; ++q) sc->wloc[q] = sc->wmin[q];
@@ -291,8 +258,8 @@ __global__ void save_local_limits_kernel(Scalars* sc) {
 }
 
 __global__ void reset_reduction_kernel(Scalars* sc) {
-    sc->wmin[0] = sc->wmin[1] = sc->wmin[2] = sc->wmin[3] = order_key(1e300);
-    sc->umax = order_key(0.0);
+    clear_limits(sc);
+    sc->wmin[3] = order_key(1e300);
 }
 
 cudaError_t launch_step_begin(const Physics& ph, Scalars* sc, cudaStream_t st) {

@@ -75,6 +75,13 @@ struct Boundary {
     int half_nx;      // NX/2 for ITCON 4
 };
 
+// The thresholds as float coefficients for one cell's comparisons (fold_dt_filtered).
+struct DtBounds {
+    float u;           // Mach term: skipped cells have |m|^2 < u T rho^2 (0: skip nothing)
+    float a1, a2, a3;  // CFL: dd^2 rho^2 > a1 |m|^2 + a2 T rho^2 + a3 |B|^2 rho
+    float q2, q3;      // conduction, viscosity: dd^2 rho > q2 rkapa, dd^2 rho > q3
+};
+
 // Device-resident scalars and the running dt reduction (ordered-integer keys).
 struct Scalars {
     double dt, timc, timt, timi, umach, tb;
@@ -86,18 +93,19 @@ struct Scalars {
     unsigned long long wmin[4];  // keys of min(ww1), min(ww2), min(ww3), min(vv)
     unsigned long long umax;     // key of max(ogamma*uu/tt)
     double mass, energy;         // diagnostics (r3d_gpu_totals)
-    // Threshold filter of the third stage's limits (fold_dt_filtered): on whole-domain handles,
-    // cells whose estimated ww1 exceeds thr_w1 and whose Mach term is below thr_um skip the exact
-    // evaluation.  step_begin sets the thresholds from the previous limits widened by
-    // thr_margin; step_end sets refold when the filtered minimum/maximum fails the check, and
-    // the limits are then evaluated again over the whole state.
+    // Threshold filter of the third stage's limits (fold_dt_filtered): a cell is skipped when
+    // bounds derived from its values put its CFL, conduction and viscosity limits above thr_w[0..2]
+    // and its Mach term below thr_um.  step_begin sets the thresholds from the previous limits
+    // widened by thr_margin; step_end sets refold when a filtered minimum or the maximum fails the
+    // check, and the limits are then evaluated again over the whole state.
     int thr_on;
     int thr_local;  // a slab: thresholds from its own limits (wloc, uloc), saved before they are
                     // combined with the other slabs' (the check at step_end is then per slab)
     int refold;
     int refolds;  // number of re-evaluations since the upload (diagnostic)
     double thr_margin;
-    double thr_w1, thr_um;
+    double thr_w[3], thr_um;
+    DtBounds bnd;
     unsigned long long wloc[4], uloc;  // this slab's limit keys before the cross-slab reduction
 };
 

@@ -42,55 +42,48 @@ __device__ __forceinline__ bool est_window(double x) {
     return (unsigned)__double2hiint(x) - 0x3e100000u < 0x03d00000u;
 }
 
-// Fold one cell's time-step limits into running minima m1..m4 and maximum mu.  The cheap limits
-// (ww2, ww3, vv: products of the cell's spacing and density) are folded exactly.  The costly
-// FP64 ww1 = dd/sqrt(c^2) and Mach term (a reciprocal, two divisions, two square roots) are
-// evaluated only for cells that can change m1 or mu: float estimates of both, with relative
-// error below 2^-17 (at most thirty float operations on positive quantities, each correctly
-// rounded or within 2 ulp, inputs in the est_window range), are compared under a 2^-12 margin
-// with b1 = min(m1, t1) and bu = max(mu, tu).  A cell is skipped only when its estimates are
-// clearly worse than both bounds; cells outside the window, with a non-finite estimate, or
-// while bu <= 2^-40 (where float underflow voids the bound on the Mach term) are evaluated.
-// With t1 = +huge and tu = 0 the running values equal those of folding the FP64 values of every
-// cell.  With thresholds t1, tu the skipped cells have ww1 > t1 and Mach term < tu, so the
-// folded limits over the whole domain are exact whenever the final minimum is <= t1 and the
-// final maximum is >= tu (checked by step_end_kernel, which requests a full re-evaluation
-// otherwise).  Expressions and operation order of the exact path are those of dt_terms.
-template <bool KC, bool MHD>
-__device__ __forceinline__ void fold_dt_filtered(const Physics& ph, double ru, double rv,
-                                                 double rw, double ro, double tt, double b2sum,
-                                                 double dd, double rkap, double t1, double tu,
-                                                 double& m1, double& m2, double& m3, double& m4,
-                                                 double& mu) {
-    m2 = fold_min(m2, KC ? 0.5 * dd * dd * ph.repr * ph.cv * ro                  // src/step.cpp:192-193
-                         : 0.5 * dd * dd * ph.repr * ph.cv * ro / rkap);
-    m3 = fold_min(m3, 0.375 * dd * dd * ph.re * ro);                            // src/step.cpp:194
-    if constexpr (MHD) m4 = fold_min(m4, 0.5 * dd * dd * ph.rm);
-    const float rof = (float)ro, ttf = (float)tt;
-    const float ruf = (float)ru, rvf = (float)rv, rwf = (float)rw;
-    const float rf = __fdividef(1.0f, rof);
-    const float uuf = (ruf * ruf + rvf * rvf + rwf * rwf) * rf * rf;
-    const float umf = __fdividef(ph.ogamma_f * uuf, ttf);
-    const float gtf = ph.gamma_f * ttf;
-    float c2f;
-    // square roots as x * rsqrt(x) (2 ulp each; 0 for x == 0)
-    auto sqrt_est = [](float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; };
-    if constexpr (MHD) {
-        const float b2f = (float)b2sum * ph.obeta_f * rf;
-        c2f = uuf + gtf + b2f + 2.0f * sqrt_est(uuf * (gtf + b2f));
-    } else {
-        c2f = uuf + gtf + 2.0f * sqrt_est(uuf * gtf);
-    }
-    const float w1f = (float)dd * rsqrtf(c2f);
-    const double b1 = (t1 < m1) ? t1 : m1;
-    const double bu = (mu < tu) ? tu : mu;
-    const bool ok = est_window(ro) && est_window(tt) && est_window(dd);
-    const bool skip_um = ok && bu > 0x1p-40 && (double)umf * (1.0 + 1.0 / 4096.0) < bu;
-    const bool skip_w1 = ok && (double)w1f * (1.0 - 1.0 / 4096.0) > b1;
-    if (skip_um && skip_w1) return;
+// The plane-independent part of a cell's dd = min(ddx, ddy, ddz) for the filter: min(ddx, ddy)^2 in
+// float, 0 (no cell is skipped) when it is outside the window of the estimates.
+__device__ __forceinline__ float dd2_est(double dd) {
+    return est_window(dd) ? (float)dd * (float)dd : 0.0f;
+}
+
+// Fold one cell's time-step limits into running minima m1..m3 and maximum mu, evaluating them (a
+// reciprocal, two divisions, two square roots and some fifteen products in FP64) only for cells
+// that can matter.  With m = rho u, the limits are
+//     Mach term  um = |m|^2 / (gamma T rho^2)
+//     CFL        w1 = dd / (|u| + c),  c^2 = gamma T (+ obeta |B|^2 / rho)
+//     conduction w2 = 0.5 repr cv dd^2 rho / rkapa,   viscosity  w3 = 0.375 re dd^2 rho
+// and (|u| + c)^2 <= (1 + 1/s) |u|^2 + (1 + s) c^2 for any s > 0 (2 |u| c <= |u|^2/s + s c^2; step_begin
+// takes s^2 = the Mach term's threshold, where the bound is tight).  So a cell has um < thr_um and
+// every limit above its threshold when |m|^2 < u T rho^2, dd^2 rho^2 > a1 |m|^2 + a2 T rho^2 +
+// a3 |B|^2 rho and dd^2 rho > max(q2 rkapa, q3) - products and sums of positive quantities, formed in
+// float from correctly rounded inputs in 2^-30 .. 2^30 with a relative error below 2^-19, against
+// coefficients that step_begin widens by 2^-10.  A non-finite value fails a comparison and the
+// cell is evaluated.  The folded limits over the whole domain are exact whenever the final minima
+// are <= and the maximum >= their thresholds (checked by step_end, which requests a full
+// re-evaluation otherwise).  The resistive limit depends on the grid alone: the whole-state
+// evaluation after an upload leaves its minimum, which no step clears.
+// dd2: min(dd2_est(min(ddx, ddy)), dd2_est(ddz)); qk: max(q2 rkapa, q3); dd evaluates min_of3(...).
+__device__ __forceinline__ bool dt_skip(const DtBounds& B, float ru, float rv, float rw, float ro, float tt,
+                                        float bcfl, float dd2, float qk) {
+    const float msq = ru * ru + rv * rv + rw * rw, r2 = ro * ro, tr2 = tt * r2;
+    return ro >= 0x1p-30f && ro < 0x1p30f && tt >= 0x1p-30f && tt < 0x1p30f && msq < B.u * tr2 &&
+           dd2 * r2 > B.a1 * msq + B.a2 * tr2 + bcfl && dd2 * ro > qk;
+}
+
+template <bool KC, bool MHD, class DD>
+__device__ __forceinline__ void fold_dt_filtered(const Physics& ph, const DtBounds& B, double ru, double rv, double rw,
+                                                 double ro, double tt, double b2sum, float dd2, float qk, DD dd,
+                                                 double rkap, double& m1, double& m2, double& m3, double& mu) {
+    const float rof = (float)ro;
+    if (dt_skip(B, (float)ru, (float)rv, (float)rw, rof, (float)tt, MHD ? B.a3 * ((float)b2sum * rof) : 0.0f, dd2, qk))
+        return;
     double w1, w2, w3, w4, um;
-    dt_terms<KC>(ph, ru, rv, rw, ro, tt, MHD ? b2sum : 0.0, dd, rkap, w1, w2, w3, w4, um);
+    dt_terms<KC>(ph, ru, rv, rw, ro, tt, MHD ? b2sum : 0.0, dd(), rkap, w1, w2, w3, w4, um);
     m1 = fold_min(m1, w1);
+    m2 = fold_min(m2, w2);
+    m3 = fold_min(m3, w3);
     mu = fold_max(mu, um);
 }
 
@@ -167,6 +160,74 @@ __device__ __forceinline__ void put_periodic(T* f, int64_t base, const Geometry&
     if (gi >= 0) f[base + (int64_t)j * g.pitch + gi] = v;
     if (gj >= 0) f[base + (int64_t)gj * g.pitch + i] = v;
     if (gi >= 0 && gj >= 0) f[base + (int64_t)gj * g.pitch + gi] = v;
+}
+
+// Start of a step (src/step.cpp:133-141, 224-229): dt = sff*min(...).
+__device__ __forceinline__ double step_dt(const Physics& ph, const Scalars* sc) {
+    const double w0 = order_value(sc->wmin[0]), w1 = order_value(sc->wmin[1]);
+    const double w2 = order_value(sc->wmin[2]), w3 = order_value(sc->wmin[3]);
+    double m = (w1 < w0) ? w1 : w0;
+    m = (w2 < m) ? w2 : m;
+    if (ph.lmag) m = (w3 < m) ? w3 : m;
+    return ph.sff * m;
+}
+
+// The rest of the start of a step, once per step: dt, umach = sqrt(max(...)) and the thresholds of
+// the filtered fold: the previous limits widened by the margin (a margin < 0 forces the
+// re-evaluation path; thr_on == 0 skips nothing); a slab takes its own limits, so that its check
+// at the step's end makes its own fold exact.
+__device__ __forceinline__ void step_begin(const Physics& ph, Scalars* sc) {
+    sc->dt = step_dt(ph, sc);
+    const double u = order_value(sc->umax);
+    sc->umach = sqrt(u);
+    double t[3];
+    for (int q = 0; q < 3; ++q) {
+        t[q] = order_value(sc->thr_local ? sc->wloc[q] : sc->wmin[q]) * (1.0 + sc->thr_margin);
+        sc->thr_w[q] = sc->thr_on ? t[q] : 1e308;
+    }
+    const double tu = (sc->thr_local ? order_value(sc->uloc) : u) * (1.0 - sc->thr_margin);
+    sc->thr_um = sc->thr_on ? tu : 0.0;
+    DtBounds B{};  // u == 0: every cell is evaluated
+    const double s = sqrt(tu), wide = 1.0 + 0x1p-10, t2 = t[0] * t[0] * wide;
+    const double q2 = t[1] * wide / (0.5 * ph.repr * ph.cv), q3 = t[2] * wide / (0.375 * ph.re);
+    // thresholds far outside the range of any flow (and NaN) would leave float's range
+    if (sc->thr_on && tu > 0x1p-40 && tu < 0x1p40 && t[0] > 0x1p-30 && t[0] < 0x1p30 && q2 > 0x1p-60 && q2 < 0x1p60 &&
+        q3 > 0x1p-60 && q3 < 0x1p60) {
+        B.u = (float)(tu * ph.gamma / wide);
+        B.a1 = (float)(t2 * (1.0 + 1.0 / s));
+        B.a2 = (float)(t2 * (1.0 + s) * ph.gamma);
+        B.a3 = (float)(t2 * (1.0 + s) * ph.obeta);
+        B.q2 = (float)q2;
+        B.q3 = (float)q3;
+    }
+    sc->bnd = B;
+}
+
+// The limits a step folds anew (all but the resistive one, wmin[3]: it depends on the grid alone).
+__device__ __forceinline__ void clear_limits(Scalars* sc) {
+    sc->wmin[0] = sc->wmin[1] = sc->wmin[2] = order_key(1e300);
+    sc->umax = order_key(0.0);
+}
+
+// End of a step: nit, timc, timt (src/step.cpp:254-256).  check != 0 (after a full step on a
+// handle with the threshold filter): the skipped cells have limits > thr_w and a Mach term < thr_um,
+// so the folded limits are exact iff the minima found are <= thr_w and the maximum >= thr_um;
+// otherwise clear them and request the full evaluation (dt_full_kernel with only_refold).  The
+// keys are read past L1: the third stage's other CTAs wrote them.
+__device__ __forceinline__ void step_end(Scalars* sc, int check) {
+    sc->nit += 1;
+    sc->timc += sc->dt;
+    sc->timt = sc->timi + sc->timc;
+    int refold = 0;
+    if (check && sc->thr_on) {
+        refold = !(order_value(__ldcg(&sc->umax)) >= sc->thr_um);
+        for (int q = 0; q < 3; ++q) refold |= !(order_value(__ldcg(&sc->wmin[q])) <= sc->thr_w[q]);
+        if (refold) {
+            sc->refolds += 1;
+            clear_limits(sc);
+        }
+    }
+    sc->refold = refold;
 }
 
 __device__ __forceinline__ uint64_t global_ns() {

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(Sh::NT, STAGE == 2 ? Sh::ctas_s2 : Sh::ctas)
     float* der = reinterpret_cast<float*>(smem + Sh::raw_bytes);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Sh::raw_bytes + Sh::der_bytes);
     __shared__ int s_abort;
-    __shared__ double s_thr[2];  // third stage: thresholds of the dt filter (thr_w1, thr_um)
+    __shared__ DtBounds s_bnd;  // third stage: bounds of the filtered dt fold
 
     const int tid = threadIdx.x;
     const int ty = tid / PXN, px = tid % PXN;
@@ -165,10 +165,7 @@ __global__ void __launch_bounds__(Sh::NT, STAGE == 2 ? Sh::ctas_s2 : Sh::ctas)
     if (tid == 0) {
         s_abort = (*(volatile int*)&sc->err != kErrNone) ? 2 : 0;
         tx_extra = sc->tx_extra;
-        if (STAGE == 2) {
-            s_thr[0] = sc->thr_w1;
-            s_thr[1] = sc->thr_um;
-        }
+        if (STAGE == 2) s_bnd = sc->bnd;
         for (int b = 0; b < NRAW; ++b) mbar_init(&bars[b], 1);
         fence_mbar_init();
     }
@@ -188,8 +185,9 @@ __global__ void __launch_bounds__(Sh::NT, STAGE == 2 ? Sh::ctas_s2 : Sh::ctas)
     const v2 cg = B2((float)(ph.gam[STAGE] * dt));
     const v2 cz = B2((STAGE < 2) ? (float)(ph.zeta[STAGE + 1] * dt) : 0.0f);
     const int ia = act0 ? i : 1, ib = act1 ? i + 1 : ia, ja = act0 ? j : 1;
-    const double dxy0 = (L.ddy[ja] < L.ddx[ia]) ? L.ddy[ja] : L.ddx[ia];  // the plane-independent part of dd
-    const double dxy1 = (L.ddy[ja] < L.ddx[ib]) ? L.ddy[ja] : L.ddx[ib];
+    // third stage: estimates of min(ddx, ddy)^2 for the dt filter
+    const float dd20 = dd2_est((L.ddy[ja] < L.ddx[ia]) ? L.ddy[ja] : L.ddx[ia]);
+    const float dd21 = dd2_est((L.ddy[ja] < L.ddx[ib]) ? L.ddy[ja] : L.ddx[ib]);
     const v2 cx = make_float2((float)(ph.hx * L.dxxdx[ia]), (float)(ph.hx * L.dxxdx[ib]));  // d/dx
     const v2 cx1 = make_float2((float)(ph.hx * L.d2xxdx2[ia]), (float)(ph.hx * L.d2xxdx2[ib]));
     const v2 cx2 = make_float2((float)(ph.h2x * L.dxxdx[ia] * L.dxxdx[ia]), (float)(ph.h2x * L.dxxdx[ib] * L.dxxdx[ib]));
@@ -392,21 +390,27 @@ __global__ void __launch_bounds__(Sh::NT, STAGE == 2 ? Sh::ctas_s2 : Sh::ctas)
                 }
             }
         }
-        if (STAGE == 2 && !edge) {  // dt limits, FP64 values on full state (filtered)
-            const double rk = bg.r[k], tk = bg.t[k];
+        if (STAGE == 2 && !edge) {  // dt limits: the filter in FP32, FP64 values on the full state
+            const float dd2z = dd2_est(L.ddz[k]), qk = fmaxf(s_bnd.q2 * kb4.w, s_bnd.q3);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (h == 1 && !act1) break;
-                const double dxy = h ? dxy1 : dxy0;
-                const double dd = (L.ddz[k] < dxy) ? L.ddz[k] : dxy;  // min_of3(ddx, ddy, ddz)
                 const float a0 = h ? xn[0].y : xn[0].x, a1 = h ? xn[1].y : xn[1].x, a2 = h ? xn[2].y : xn[2].x;
-                const double ro = rk + (double)(h ? xn[3].y : xn[3].x), tt = tk + (double)(h ? xn[4].y : xn[4].x);
-                if (ph.kappa_const)  // rkapa == 1 on every plane: x/rkapa == x, no division
-                    fold_dt_filtered<true, false>(ph, a0, a1, a2, ro, tt, 0.0, dd, 1.0, s_thr[0], s_thr[1], m1,
-                                                  m2, m3, m4, mu);
-                else
-                    fold_dt_filtered<false, false>(ph, a0, a1, a2, ro, tt, 0.0, dd, L.rkapa[k], s_thr[0],
-                                                   s_thr[1], m1, m2, m3, m4, mu);
+                const float a3 = h ? xn[3].y : xn[3].x, a4 = h ? xn[4].y : xn[4].x;
+                const float rof = bg.rf[k] + a3, ttf = bg.tf[k] + a4;
+                if (!dt_skip(s_bnd, a0, a1, a2, rof, ttf, 0.0f, fminf(h ? dd21 : dd20, dd2z), qk)) {
+                    double w1, w2, w3, w4, um;
+                    const double dd = min_of3(L.ddx[i + h], L.ddy[j], L.ddz[k]);
+                    const double ro = bg.r[k] + (double)a3, tt = bg.t[k] + (double)a4;
+                    if (ph.kappa_const)  // rkapa == 1 on every plane: x/rkapa == x, no division
+                        dt_terms<true>(ph, a0, a1, a2, ro, tt, 0.0, dd, 1.0, w1, w2, w3, w4, um);
+                    else
+                        dt_terms<false>(ph, a0, a1, a2, ro, tt, 0.0, dd, L.rkapa[k], w1, w2, w3, w4, um);
+                    m1 = fold_min(m1, w1);
+                    m2 = fold_min(m2, w2);
+                    m3 = fold_min(m3, w3);
+                    mu = fold_max(mu, um);
+                }
             }
         }
 #undef RX_

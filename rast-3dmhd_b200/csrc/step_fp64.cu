@@ -166,8 +166,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
     double* der = reinterpret_cast<double*>(smem + S::raw_bytes);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::raw_bytes + S::der_bytes);
     __shared__ int s_abort;
-    __shared__ int s_filter;     // third stage: threshold-filtered dt fold (Scalars::thr_on)
-    __shared__ double s_thr[2];  // its thresholds thr_w1, thr_um
+    __shared__ DtBounds s_bnd;  // third stage: bounds of the filtered dt fold
 
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
     const int i0 = 1 + blockIdx.x * TX, j0 = 1 + blockIdx.y * TY;
@@ -240,11 +239,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
         // a CTA that finds an earlier timeout recorded leaves before issuing any copy
         s_abort = (*(volatile int*)&sc->err != kErrNone) ? 2 : 0;
         tx_extra = sc->tx_extra;
-        if (STAGE == 2) {
-            s_filter = sc->thr_on;
-            s_thr[0] = sc->thr_w1;
-            s_thr[1] = sc->thr_um;
-        }
+        if (STAGE == 2) s_bnd = sc->bnd;
         for (int b = 0; b < NRAW; ++b) mbar_init(&bars[b], 1);
         fence_mbar_init();
     }
@@ -288,7 +283,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
     // per row c of the thread: activity, y metrics, column offset
     bool actv[CPT];
     int colv[CPT];
-    double dxyv[CPT];  // third stage: min(ddx[i], ddy[j]), the plane-independent part of dd
+    float dd2v[CPT];  // third stage: estimate of min(ddx[i], ddy[j])^2 for the dt filter
 #pragma unroll
     for (int c = 0; c < CPT; ++c) {
         const int j = jr + c;
@@ -296,7 +291,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
         colv[c] = ((j <= g.npy) ? j : 1) * PX + ia;
         if (STAGE == 2) {
             const int ja = (j <= g.npy) ? j : 1;
-            dxyv[c] = (L.ddy[ja] < L.ddx[ia]) ? L.ddy[ja] : L.ddx[ia];
+            dd2v[c] = dd2_est((L.ddy[ja] < L.ddx[ia]) ? L.ddy[ja] : L.ddx[ia]);
         }
     }
 
@@ -701,22 +696,11 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
                 }
             }
             if (STAGE == 2 && !EMIT && !edge) {  // the adjoint's recompute needs no limits
-                const double dd = (L.ddz[k] < dxyv[c]) ? L.ddz[k] : dxyv[c];  // min_of3(ddx, ddy, ddz)
                 double b2sum = 0.0;
                 if constexpr (MHD) b2sum = xn[5] * xn[5] + xn[6] * xn[6] + xn[7] * xn[7];
-                if (s_filter) {
-                    fold_dt_filtered<KC, MHD>(ph, xn[0], xn[1], xn[2], xn[3], xn[4], b2sum, dd,
-                                              L.rkapa[k], s_thr[0], s_thr[1], m1, m2, m3, m4, mu);
-                } else {
-                    double w1, w2, w3, w4, um;
-                    dt_terms<KC>(ph, xn[0], xn[1], xn[2], xn[3], xn[4], b2sum, dd, L.rkapa[k], w1,
-                                 w2, w3, w4, um);
-                    m1 = fold_min(m1, w1);
-                    m2 = fold_min(m2, w2);
-                    m3 = fold_min(m3, w3);
-                    m4 = fold_min(m4, w4);
-                    mu = fold_max(mu, um);
-                }
+                fold_dt_filtered<KC, MHD>(ph, s_bnd, xn[0], xn[1], xn[2], xn[3], xn[4], b2sum, fminf(dd2v[c], dd2_est(L.ddz[k])),
+                                          fmaxf(KC ? s_bnd.q2 : s_bnd.q2 * (float)L.rkapa[k], s_bnd.q3),
+                                          [&] { return min_of3(L.ddx[i], L.ddy[j], L.ddz[k]); }, L.rkapa[k], m1, m2, m3, mu);
             }
           }
         }
