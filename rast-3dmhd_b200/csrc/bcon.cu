@@ -20,84 +20,11 @@ __global__ void __launch_bounds__(256) bcon_kernel(Geometry g, Physics ph, Lines
     __shared__ double red[5 * 8];
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    const bool active = (i <= g.npx) && (j <= g.npy);
+    const int side = blockIdx.z;  // 0 top, 1 bottom
     double m1 = 1e300, m2 = 1e300, m3 = 1e300, m4 = 1e300, mu = 0.0;
-    if (active) {
-        double* ru = fs.xout[0];
-        double* rv = fs.xout[1];
-        double* rw = fs.xout[2];
-        double* ro = fs.xout[3];
-        double* tt = fs.xout[4];
-        const double c13 = ph.c13, c23 = ph.c23, c43 = ph.c43;
-        const int64_t P = g.plane, row = (int64_t)j * g.pitch + i;
-        // top, k = 1 (src/bcon.cpp:27-98); a z slab that does not hold the domain's top
-        // plane has a neighbour's ghost plane there instead
-        if (g.top_edge) {
-            const int64_t n = P + row;
-            const double ro1 = ro[n], ro2 = ro[n + P], ro3 = ro[n + 2 * P];
-            const double u = ro1 * (c43 * ru[n + P] / ro2 - c13 * ru[n + 2 * P] / ro3);
-            const double v = ro1 * (c43 * rv[n + P] / ro2 - c13 * rv[n + 2 * P] / ro3);
-            double t;
-            switch (b.top_mode) {
-                case 0: t = 1.0; break;
-                case 1: t = c43 * tt[n + P] - c13 * tt[n + 2 * P] - c23 * b.dz_top * b.theta; break;
-                case 2: t = 1.0 - (1.0 - b.tpr) * L.plume_x[i] / b.hh * L.plume_y[j] / b.hh; break;
-                case 3:
-                    t = c43 * tt[n + P] - c13 * tt[n + 2 * P] -
-                        c23 * b.dz_top * (b.theta - (b.theta - b.tpr) * L.plume_x[i] / b.hh * L.plume_y[j] / b.hh);
-                    break;
-                case 5: t = tt[n]; break;  // itcon 3: the stage's value stands
-                default: t = (i <= b.half_nx) ? 1.0 - b.tp : 1.0; break;
-            }
-            put_periodic(ru, P, g, i, j, u);
-            put_periodic(rv, P, g, i, j, v);
-            put_periodic(rw, P, g, i, j, 0.0);
-            put_periodic(tt, P, g, i, j, t);
-            double b2 = 0.0;
-            if (ph.lmag) {
-                put_periodic(fs.xout[7], P, g, i, j, 0.0);
-                const double bx = fs.xout[5][n], by = fs.xout[6][n];
-                b2 = bx * bx + by * by + 0.0 * 0.0;
-            }
-            if (with_dt) {
-                const double dd = min_of3(L.ddx[i], L.ddy[j], L.ddz[1]);
-                double w1, w2, w3, w4, um;
-                dt_terms(ph, u, v, 0.0, ro1, t, b2, dd, L.rkapa[1], w1, w2, w3, w4, um);
-                m1 = fold_min(m1, w1); m2 = fold_min(m2, w2); m3 = fold_min(m3, w3);
-                m4 = fold_min(m4, w4); mu = fold_max(mu, um);
-            }
-        }
-        // bottom, k = npz (src/bcon.cpp:104-139)
-        if (g.bot_edge) {
-            const int64_t n = (int64_t)g.npz * P + row;
-            const double ro1 = ro[n], ro2 = ro[n - P], ro3 = ro[n - 2 * P];
-            const double u = ro1 * (c43 * ru[n - P] / ro2 - c13 * ru[n - 2 * P] / ro3);
-            const double v = ro1 * (c43 * rv[n - P] / ro2 - c13 * rv[n - 2 * P] / ro3);
-            double t;
-            if (b.bottom_mode == 0)
-                t = b.tb;
-            else
-                t = c43 * tt[n - P] - c13 * tt[n - 2 * P] + c23 * b.dz_bot * b.theta / L.rkapa[g.npz];
-            const int64_t base = (int64_t)g.npz * P;
-            put_periodic(ru, base, g, i, j, u);
-            put_periodic(rv, base, g, i, j, v);
-            put_periodic(rw, base, g, i, j, 0.0);
-            put_periodic(tt, base, g, i, j, t);
-            double b2 = 0.0;
-            if (ph.lmag) {
-                put_periodic(fs.xout[7], base, g, i, j, 0.0);
-                const double bx = fs.xout[5][n], by = fs.xout[6][n];
-                b2 = bx * bx + by * by + 0.0 * 0.0;
-            }
-            if (with_dt) {
-                const double dd = min_of3(L.ddx[i], L.ddy[j], L.ddz[g.npz]);
-                double w1, w2, w3, w4, um;
-                dt_terms(ph, u, v, 0.0, ro1, t, b2, dd, L.rkapa[g.npz], w1, w2, w3, w4, um);
-                m1 = fold_min(m1, w1); m2 = fold_min(m2, w2); m3 = fold_min(m3, w3);
-                m4 = fold_min(m4, w4); mu = fold_max(mu, um);
-            }
-        }
-    }
+    // a z slab that does not hold the domain's top or bottom plane has a neighbour's ghost plane there
+    if (i <= g.npx && j <= g.npy && (side == 0 ? g.top_edge : g.bot_edge))
+        bcon_column(g, ph, L, b, fs.xout, side, i, j, with_dt != 0, m1, m2, m3, m4, mu);
     if (with_dt) reduce_dt(red, m1, m2, m3, m4, mu, sc);
 }
 
@@ -159,7 +86,7 @@ cudaError_t launch_plane_mean(const Geometry& g, const double* ro, double* rom, 
 cudaError_t launch_bcon(const Geometry& g, const Physics& ph, const Lines& L, const Boundary& b,
                         const FieldSet& fs, Scalars* sc, int with_dt, cudaStream_t st) {
     dim3 block(32, 8, 1);
-    dim3 grid((g.npx + 31) / 32, (g.npy + 7) / 8, 1);
+    dim3 grid((g.npx + 31) / 32, (g.npy + 7) / 8, 2);
     bcon_kernel<<<grid, block, 0, st>>>(g, ph, L, b, fs, sc, with_dt);
     return cudaGetLastError();
 }

@@ -162,6 +162,63 @@ __device__ __forceinline__ void put_periodic(T* f, int64_t base, const Geometry&
     if (gi >= 0 && gj >= 0) f[base + (int64_t)gj * g.pitch + gi] = v;
 }
 
+// BCON (src/bcon.cpp:12-141) of one column on the domain's top plane k = 1 (side 0, src/bcon.cpp:
+// 27-98) or bottom plane k = npz (side 1, src/bcon.cpp:104-139), ghost images included; with dt
+// the plane's time-step limits are folded as well.  Bound by latency (its loads all go out first, then
+// two chains of divisions): one thread per column and side, and one copy of the code for both sides.
+__device__ __forceinline__ void bcon_column(const Geometry& g, const Physics& ph, const Lines& L, const Boundary& b,
+                                            double* const* x, int side, int i, int j, bool dt, double& m1, double& m2,
+                                            double& m3, double& m4, double& mu) {
+    const double c13 = ph.c13, c23 = ph.c23, c43 = ph.c43;
+    const int k = side == 0 ? 1 : g.npz;
+    const int64_t d = side == 0 ? g.plane : -g.plane;
+    const int64_t base = (int64_t)k * g.plane, n = base + (int64_t)j * g.pitch + i;
+    const int64_t n1 = n + d, n2 = n1 + d;
+    const double *ru = x[0], *rv = x[1], *ro = x[3], *tt = x[4];
+    const double ro1 = __ldcg(ro + n), ro2 = __ldcg(ro + n1), ro3 = __ldcg(ro + n2);
+    const double u2 = __ldcg(ru + n1), u3 = __ldcg(ru + n2), v2 = __ldcg(rv + n1), v3 = __ldcg(rv + n2);
+    const double t1 = __ldcg(tt + n), t2 = __ldcg(tt + n1), t3 = __ldcg(tt + n2);
+    const double u = ro1 * (c43 * u2 / ro2 - c13 * u3 / ro3);
+    const double v = ro1 * (c43 * v2 / ro2 - c13 * v3 / ro3);
+    const int mode = side == 0 ? b.top_mode : (b.bottom_mode == 0 ? 6 : 7);
+    const double lin = c43 * t2 - c13 * t3;  // modes 1, 3, 7
+    double t;
+    if (mode == 2 || mode == 3) {  // plume: * plume_x / hh * plume_y / hh
+        double f = (mode == 2 ? 1.0 - b.tpr : b.theta - b.tpr) * L.plume_x[i];
+        if (b.hh != 1.0) f = f / b.hh;
+        f = f * L.plume_y[j];
+        if (b.hh != 1.0) f = f / b.hh;
+        t = mode == 2 ? 1.0 - f : lin - c23 * b.dz_top * (b.theta - f);
+    } else if (mode == 1) {
+        t = lin - c23 * b.dz_top * b.theta;
+    } else if (mode == 7) {
+        t = lin + c23 * b.dz_bot * b.theta / L.rkapa[g.npz];
+    } else {
+        // constant, itcon 3 (the stage's value stands), half-domain, constant bottom temperature
+        t = mode == 0 ? 1.0 : (mode == 5 ? t1 : (mode == 6 ? b.tb : ((i <= b.half_nx) ? 1.0 - b.tp : 1.0)));
+    }
+    put_periodic(x[0], base, g, i, j, u);
+    put_periodic(x[1], base, g, i, j, v);
+    put_periodic(x[2], base, g, i, j, 0.0);
+    put_periodic(x[4], base, g, i, j, t);
+    double b2 = 0.0;
+    if (ph.lmag) {
+        put_periodic(x[7], base, g, i, j, 0.0);
+        const double bx = __ldcg(x[5] + n), by = __ldcg(x[6] + n);
+        b2 = bx * bx + by * by + 0.0 * 0.0;
+    }
+    if (dt) {
+        const double dd = min_of3(L.ddx[i], L.ddy[j], L.ddz[k]);
+        double w1, w2, w3, w4, um;
+        dt_terms(ph, u, v, 0.0, ro1, t, b2, dd, L.rkapa[k], w1, w2, w3, w4, um);
+        m1 = fold_min(m1, w1);
+        m2 = fold_min(m2, w2);
+        m3 = fold_min(m3, w3);
+        m4 = fold_min(m4, w4);
+        mu = fold_max(mu, um);
+    }
+}
+
 // Start of a step (src/step.cpp:133-141, 224-229): dt = sff*min(...).
 __device__ __forceinline__ double step_dt(const Physics& ph, const Scalars* sc) {
     const double w0 = order_value(sc->wmin[0]), w1 = order_value(sc->wmin[1]);
