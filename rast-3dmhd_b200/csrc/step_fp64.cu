@@ -71,8 +71,9 @@ constexpr int NDER = 4;
 // the derived ring (1/rho of the thread's own cells stays in registers; P = rho*T is formed
 // where it is used, the product the reference stores).  MHD keeps the 4-slot raw ring and the
 // derived u, v, w, P, 1/rho.  Both prefetch the RK accumulators of the next plane into L2 and
-// load a plane's accumulators during the plane - hydro after its fluxes, just before the stage
-// update, MHD before its derive phase - which takes fewer registers than holding the next
+// load a plane's accumulators during the plane - hydro the first row's before its fluxes and the
+// second row's after them, just before the stage update (504x504x128 on B200: 3826 -> 3804 us per step
+// against both rows after; both before would spill), MHD before its derive phase - which takes fewer registers than holding the next
 // plane's values in registers (hydro: 40, and no spills).  Measured on B200 at 1965 MHz:
 // 504x504x512 hydro 15.45 -> 14.9 ms per step, 126x126x256 MHD 0.946 -> 0.901 ms (0.936 with
 // the hydro placement); a prefetch two planes ahead was slower in every placement.
@@ -175,6 +176,8 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
     const int i = i0 + tx, jr = j0 + ty * CPT;  // the thread's column and first row
 
     constexpr bool LEAN = Ring<MHD>::lean;
+    // hydro: rows of the thread whose accumulators are loaded before the fluxes, the others after
+    constexpr int ZE = (LEAN && STAGE > 0 && CPT > 1) ? 1 : 0;
     constexpr int NRAW = Ring<MHD>::nraw;
     // the thread's own cells in the halo tile (row c of the thread: halo row ty*CPT + c + 1)
     const int own0 = (ty * CPT + 1) * SX + tx + 1;
@@ -312,10 +315,10 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
 #pragma unroll
             for (int c = 0; c < CPT; ++c) riq[c] = rin[c];
         }
-        if constexpr (!LEAN) {
-            // MHD: this plane's accumulators, issued before the derive phase and the barrier
+        auto load_z = [&](int c0, int c1) {
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
+                if (c < c0 || c >= c1) continue;
 #pragma unroll
                 for (int f = 0; f < NF; ++f) zq[c][f] = 0.0;
                 if (STAGE > 0 && actv[c]) {
@@ -323,7 +326,8 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
                     for (int f = 0; f < NF; ++f) zq[c][f] = fs.z[f][k * PL + colv[c]];
                 }
             }
-        }
+        };
+        if constexpr (!LEAN) load_z(0, CPT);  // MHD: issued before the derive phase and the barrier
         if (!derive(k + 1)) s_abort = 1;
         __syncthreads();
         if (s_abort) break;
@@ -344,6 +348,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
 #define P0_(DX, DY) (LEAN ? RW_(r0, R_RO, DX, DY) * RW_(r0, R_TT, DX, DY) : DV_(d0, D_P, DX, DY))
 #define PP_ (LEAN ? RW_(rp, R_RO, 0, 0) * RW_(rp, R_TT, 0, 0) : DV_(dp, D_P, 0, 0))
 #define PM_ (LEAN ? cm[c][R_RO] : DV_(dm, D_P, 0, 0))  // lean: cm[.][R_RO] carries P
+        if constexpr (LEAN) load_z(0, ZE);
         const double tmpz = L.tmpz[k];
         const bool edge = (k == 1 && g.top_edge) || (k == g.npz && g.bot_edge);
         // right-hand sides of the thread's cells: all rows first, so that their independent
@@ -650,18 +655,10 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
             }
         }
         if constexpr (LEAN) {
-            // hydro: this plane's accumulators (prefetched into L2 a plane earlier), loaded after
+            // hydro: the other rows' accumulators (prefetched into L2 a plane earlier), loaded after
             // the fluxes; the compiler barrier keeps the loads from being hoisted into them
             asm volatile("" ::: "memory");
-#pragma unroll
-            for (int c = 0; c < CPT; ++c) {
-#pragma unroll
-                for (int f = 0; f < NF; ++f) zq[c][f] = 0.0;
-                if (STAGE > 0 && actv[c]) {
-#pragma unroll
-                    for (int f = 0; f < NF; ++f) zq[c][f] = fs.z[f][k * PL + colv[c]];
-                }
-            }
+            load_z(ZE, CPT);
         }
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
