@@ -338,10 +338,13 @@ void recompute_step(r3d_gpu* g, Adjoint* A, const unsigned long long* key, const
     double* out[3] = {A->S[1], A->S[2], dst};
     for (int s = 0; s < 3; ++s) {
         r3dk::FieldSet fs = stage_fields(A, s, in[s], out[s]);
-        cuda_ok(r3dk::launch_stage_fp64(s, state_maps(g, A, in[s]), g->geo, g->ph, g->lines, fs, A->asc, g->depth,
+        // (the EMIT stages have no single-wave form)
+        const r3dk::StageTail tail = emit ? r3dk::StageTail{} : stage_tail(g, r3dk::kTailBcon);
+        cuda_ok(r3dk::launch_stage_fp64(s, state_maps(g, A, in[s]), g->geo, g->ph, g->lines, fs, A->asc, g->depth, tail,
                                         g->stream, emit),
                 "adjoint recompute stage");
-        cuda_ok(r3dk::launch_bcon(g->geo, g->ph, g->lines, g->bnd, fs, A->asc, 0, g->stream), "adjoint bcon");
+        if (!tail.flags)
+            cuda_ok(r3dk::launch_bcon(g->geo, g->ph, g->lines, g->bnd, fs, A->asc, 0, g->stream), "adjoint bcon");
     }
 }
 

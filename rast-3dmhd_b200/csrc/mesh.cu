@@ -71,9 +71,9 @@ void reduce(r3d_mesh* m) {
 
 void mesh_step(r3d_mesh* m, int nstages) {
     reduce(m);
-    for (r3d_gpu* g : m->slabs) enqueue_step_begin(g);
+    for (r3d_gpu* g : m->slabs) enqueue_step_begin(g, nstages);
     for (int s = 0; s < nstages; ++s) {
-        for (r3d_gpu* g : m->slabs) enqueue_stage(g, s);
+        for (r3d_gpu* g : m->slabs) enqueue_stage(g, s, nstages);
         exchange(m);
     }
     for (r3d_gpu* g : m->slabs) enqueue_step_end(g, nstages);

@@ -75,6 +75,18 @@ struct Boundary {
     int half_nx;      // NX/2 for ITCON 4
 };
 
+// The single-wave form of a stage launch (TAIL): the stage does what follows it as well, so that a
+// step on a small grid is three launches and the conditional dt_full.  BCON on the domain's top and
+// bottom planes is run by the CTA that completes the last of the three planes it reads (edge_cnt
+// counts them, two counters per column tile); the first stage forms the step's dt and thresholds
+// (kTailBegin); the third ends the step (kTailEnd), in the launch's last CTA.
+enum { kTailBcon = 1, kTailBegin = 2, kTailEnd = 4 };
+struct StageTail {
+    Boundary bnd;
+    int flags;  // 0: a plain stage launch
+    unsigned int* edge_cnt;
+};
+
 // The thresholds as float coefficients for one cell's comparisons (fold_dt_filtered).
 struct DtBounds {
     float u;           // Mach term: skipped cells have |m|^2 < u T rho^2 (0: skip nothing)
@@ -107,6 +119,7 @@ struct Scalars {
     double thr_w[3], thr_um;
     DtBounds bnd;
     unsigned long long wloc[4], uloc;  // this slab's limit keys before the cross-slab reduction
+    unsigned int ticket;  // CTAs of a TAIL third stage that are done (wraps to 0 with the last)
 };
 
 // Total order on doubles as unsigned keys: key(a) < key(b) iff a < b (NaN excluded).

@@ -9,8 +9,9 @@
 //    hydro instead of the reference's 28 (F, UU.., WW1..3 and the rho snapshot are never
 //    stored);
 //  * dt, umach, nit, timc, timt live on the device; a step is 9 kernel launches (step_begin,
-//    3 x (stage, BCON), step_end, the conditional dt_full) with no host round trip (the reference copies three full arrays to the host per step for dt,
-//    src/gpu.cpp:790-823).
+//    3 x (stage, BCON), step_end, the conditional dt_full), 4 on small grids, whose stages run BCON
+//    and the bookkeeping themselves, with no host round trip (the reference copies three full
+//    arrays to the host per step for dt, src/gpu.cpp:790-823).
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -497,76 +498,105 @@ void launch_plane_mean(r3d_gpu* g, const FieldSet& fs) {
             "plane_mean");
 }
 
-// Queue one step (nstages substages) on the device.
-void enqueue_step_begin(r3d_gpu* g) {
-    Range r("r3d.step_begin");
+r3dk::StageTail stage_tail(const r3d_gpu* g, int flags) {
+    r3dk::StageTail t{};
+    if (!g->tail) return t;
+    t.bnd = g->bnd;
+    t.edge_cnt = g->edge_cnt;
+    t.flags = flags;
+    return t;
+}
+
+// Stage s of a step of nstages (1 or 2: a partial step, whose bookkeeping is separate) and, unless
+// the stage's tail runs it, BCON.  Returns the launches made.
+int stage_and_bcon(r3d_gpu* g, int s, int nstages, Timer* tm) {
+    const r3dk::StageTail tail =
+        stage_tail(g, r3dk::kTailBcon | (nstages < 3 ? 0 : (s < 2 ? r3dk::kTailBegin : r3dk::kTailEnd)));
+    const int with_dt = s == 2 ? 1 : 0;
+    if (tm) tm->begin();
+    if (g->fp32) {
+        r3dk::FieldSet32 fs = fieldset32(g);
+        cuda_ok(r3dk::launch_stage_fp32(s, g->maps[g->cur], g->geo, g->ph, g->lines, g->bg, fs, g->dsc, g->depth, tail,
+                                        g->stream),
+                "stage32");
+        if (tm) tm->end(0);
+        if (g->tail) return 1;
+        if (tm) tm->begin();
+        cuda_ok(r3dk::launch_bcon_fp32(g->geo, g->ph, g->lines, g->bnd, g->bg, fs, g->dsc, with_dt, g->stream), "bcon32");
+    } else {
+        FieldSet fs = fieldset(g);
+        cuda_ok(r3dk::launch_stage_fp64(s, g->maps[g->cur], g->geo, g->ph, g->lines, fs, g->dsc, g->depth, tail, g->stream),
+                "stage");
+        if (tm) tm->end(0);
+        if (g->tail) return 1;
+        if (tm) tm->begin();
+        cuda_ok(r3dk::launch_bcon(g->geo, g->ph, g->lines, g->bnd, fs, g->dsc, with_dt, g->stream), "bcon");
+    }
+    if (tm) tm->end(1);
+    return 2;
+}
+
+// The step's start: host-side boundary values, the dt keys of all slabs, and dt (unless the first
+// stage's tail forms it).  Returns the launches made.
+int begin_step(r3d_gpu* g, int nstages) {
     g->bnd.tpr = plume_tpr(g);
     if (g->ph.heat_on) g->ph.heat_pre = heat_prefix(g);
     if (g->halo) halo_reduce_limits(g);
+    if (g->tail && nstages == 3) return 0;
     cuda_ok(r3dk::launch_step_begin(g->ph, g->dsc, g->stream), "step_begin");
+    return 1;
 }
 
-void enqueue_stage(r3d_gpu* g, int s) {
-    Range r("r3d.stage");
-    if (g->fp32) {
-        r3dk::FieldSet32 fs = fieldset32(g);
-        cuda_ok(r3dk::launch_stage_fp32(s, g->maps[g->cur], g->geo, g->ph, g->lines, g->bg, fs, g->dsc,
-                                        g->depth, g->stream),
-                "stage32");
-        cuda_ok(r3dk::launch_bcon_fp32(g->geo, g->ph, g->lines, g->bnd, g->bg, fs, g->dsc, s == 2 ? 1 : 0, g->stream),
-                "bcon32");
-    } else {
-        FieldSet fs = fieldset(g);
-        if (g->ph.id_mode) launch_plane_mean(g, fs);
-        cuda_ok(r3dk::launch_stage_fp64(s, g->maps[g->cur], g->geo, g->ph, g->lines, fs, g->dsc, g->depth, g->stream),
-                "stage");
-        cuda_ok(r3dk::launch_bcon(g->geo, g->ph, g->lines, g->bnd, fs, g->dsc, s == 2 ? 1 : 0, g->stream), "bcon");
+int end_step(r3d_gpu* g, int nstages) {
+    int n = 0;
+    if (!(g->tail && nstages == 3)) {
+        cuda_ok(r3dk::launch_step_end(g->dsc, g->stream, nstages == 3 ? 1 : 0), "step_end");
+        ++n;
     }
+    if (nstages < 3) {  // the next dt needs the limits of this partial-step state
+        launch_dt_full_any(g);
+        ++n;
+    } else if (g->dt_filter) {  // re-evaluation, only if the filtered limits failed the check
+        launch_dt_full_any(g, 1);
+        ++n;
+    }
+    return n;
+}
+
+// The pieces of one step for drivers that interleave several slabs.
+void enqueue_step_begin(r3d_gpu* g, int nstages) {
+    Range r("r3d.step_begin");
+    begin_step(g, nstages);
+}
+
+void enqueue_stage(r3d_gpu* g, int s, int nstages) {
+    Range r("r3d.stage");
+    if (!g->fp32 && g->ph.id_mode) launch_plane_mean(g, fieldset(g));
+    stage_and_bcon(g, s, nstages, nullptr);
     g->cur = 1 - g->cur;
 }
 
 void enqueue_step_end(r3d_gpu* g, int nstages) {
     Range r("r3d.step_end");
-    cuda_ok(r3dk::launch_step_end(g->dsc, g->stream, nstages == 3 ? 1 : 0), "step_end");
-    if (nstages < 3) launch_dt_full_any(g);  // the next dt needs the limits of this partial-step state
-    else if (g->dt_filter) launch_dt_full_any(g, 1);  // only if the filtered limits failed the check
+    end_step(g, nstages);
 }
 
 // Queue one step (nstages substages) on the device; with a Halo, the dt keys are reduced over
 // the slabs before the step and the ghost planes exchanged after every stage.
 void enqueue_step(r3d_gpu* g, int nstages, Timer& tm, int& launches, int& stage_launches) {
     Range step_range("r3d.step");
-    g->bnd.tpr = plume_tpr(g);
-    if (g->ph.heat_on) g->ph.heat_pre = heat_prefix(g);
     tm.begin();
-    if (g->halo) halo_reduce_limits(g);
-    cuda_ok(r3dk::launch_step_begin(g->ph, g->dsc, g->stream), "step_begin");
+    launches += begin_step(g, nstages);
     tm.end(2);
-    ++launches;
     for (int s = 0; s < nstages; ++s) {
         Range stage_range("r3d.stage");
-        tm.begin();
-        if (g->fp32) {
-            r3dk::FieldSet32 fs = fieldset32(g);
-            cuda_ok(r3dk::launch_stage_fp32(s, g->maps[g->cur], g->geo, g->ph, g->lines, g->bg, fs, g->dsc, g->depth, g->stream), "stage32");
-            tm.end(0);
+        if (!g->fp32 && g->ph.id_mode) {
             tm.begin();
-            cuda_ok(r3dk::launch_bcon_fp32(g->geo, g->ph, g->lines, g->bnd, g->bg, fs, g->dsc, s == 2 ? 1 : 0, g->stream), "bcon32");
-        } else {
-            FieldSet fs = fieldset(g);
-            if (g->ph.id_mode) {
-                launch_plane_mean(g, fs);
-                tm.end(2);
-                ++launches;
-                tm.begin();
-            }
-            cuda_ok(r3dk::launch_stage_fp64(s, g->maps[g->cur], g->geo, g->ph, g->lines, fs, g->dsc, g->depth, g->stream), "stage");
-            tm.end(0);
-            tm.begin();
-            cuda_ok(r3dk::launch_bcon(g->geo, g->ph, g->lines, g->bnd, fs, g->dsc, s == 2 ? 1 : 0, g->stream), "bcon");
+            launch_plane_mean(g, fieldset(g));
+            tm.end(2);
+            ++launches;
         }
-        tm.end(1);
-        launches += 2;
+        launches += stage_and_bcon(g, s, nstages, &tm);
         ++stage_launches;
         g->cur = 1 - g->cur;
         if (g->halo) {
@@ -576,15 +606,7 @@ void enqueue_step(r3d_gpu* g, int nstages, Timer& tm, int& launches, int& stage_
         }
     }
     tm.begin();
-    cuda_ok(r3dk::launch_step_end(g->dsc, g->stream, nstages == 3 ? 1 : 0), "step_end");
-    ++launches;
-    if (nstages < 3) {  // the next dt needs the limits of this (partial-step) state
-        launch_dt_full_any(g);
-        ++launches;
-    } else if (g->dt_filter) {  // re-evaluation, only if the filtered limits failed the check
-        launch_dt_full_any(g, 1);
-        ++launches;
-    }
+    launches += end_step(g, nstages);
     tm.end(2);
     g->work_ok = nstages == 3;
 }
@@ -1000,6 +1022,15 @@ r3d_gpu* create_handle(const r3d_params& pin, int z0, int nloc, cudaStream_t sha
                 const int64_t slots = (int64_t)g->num_sms * (g->fp32 ? r3dk::stage_fp32_ctas_per_sm()
                                                                      : r3dk::stage_fp64_ctas_per_sm(p->lmag, rows));
                 g->depth = (p->lmag || getenv("R3D_KCHUNK")) ? g->kchunk : launch_depth(tiles, nloc, g->kchunk, slots);
+                g->ph.id_mode = p->id;
+                // launches of at most one wave take the single-wave form
+                g->tail = tiles * ((nloc + g->depth - 1) / g->depth) <= slots &&
+                          (g->fp32 || r3dk::stage_fp64_has_tail(g->geo, g->ph));
+                if (g->tail) {
+                    g->edge_bytes = 2 * sizeof(unsigned) * (size_t)tiles;
+                    cuda_ok(cudaMalloc(&g->edge_cnt, g->edge_bytes), "cudaMalloc(counters)");
+                    g->bytes += (int64_t)g->edge_bytes;
+                }
             }
             cuda_ok(cudaStreamSynchronize(g->stream), "create");
     } catch (...) {
@@ -1027,6 +1058,7 @@ void destroy_handle(r3d_gpu* g) {
     cudaFree(g->bg_buf);
     cudaFree(g->line_buf);
     cudaFree(g->dsc);
+    cudaFree(g->edge_cnt);
     if (g->hsc) cudaFreeHost(g->hsc);
     for (int s = 0; s < 2; ++s) {
         if (g->bounce[s]) cudaFreeHost(g->bounce[s]);
@@ -1161,6 +1193,8 @@ void finish_state(r3d_gpu* g, const r3d_scalars* sc) {
     g->bnd.tb = sc->tb;
     g->host_timc = sc->timc;
     g->host_timi = sc->timi;
+    // counters that an abandoned stage may have left mid-way start over
+    if (g->tail) cuda_ok(cudaMemsetAsync(g->edge_cnt, 0, g->edge_bytes, g->stream), "reset");
     cuda_ok(r3dk::launch_reset_reduction(g->dsc, g->stream), "reset");
     launch_dt_full_any(g);
     cuda_ok(cudaStreamSynchronize(g->stream), "upload");
@@ -1337,8 +1371,8 @@ void eval_fluxes(r3d_gpu* g, int buf, double* const* out) {
         fs.z[q] = g->fscr + (size_t)(nf + q) * fe;             // accumulator, discarded
         fs.f[q] = g->fscr + (size_t)(2 * nf + q) * fe;         // F
     }
-    cuda_ok(r3dk::launch_stage_fp64(0, g->maps[buf], g->geo, g->ph, g->lines, fs, g->dsc, g->depth, g->stream,
-                                    true),
+    cuda_ok(r3dk::launch_stage_fp64(0, g->maps[buf], g->geo, g->ph, g->lines, fs, g->dsc, g->depth, r3dk::StageTail{},
+                                    g->stream, true),
             "fluxes");
     for (int q = 0; q < nf; ++q) {
         if (!out[q]) continue;

@@ -48,6 +48,9 @@ struct r3d_gpu {
     int cur = 0;
     int kchunk = 32;  // planned z-chunk depth (r3d_gpu_plan)
     int depth = 32;   // planes per CTA of its stage launches (launch_depth)
+    bool tail = false;                 // stages run in their single-wave form (r3dk::StageTail)
+    unsigned int* edge_cnt = nullptr;  // its BCON completion counters
+    size_t edge_bytes = 0;
     bool uploaded = false;
     bool work_ok = false;  // the last operation on the state was a full step (r3d_gpu_download_work)
     int64_t bytes = 0;
@@ -139,8 +142,8 @@ void pull_scalars(r3d_gpu* g, r3d_scalars* sc);
 // interleave several slabs with their ghost-plane exchanges (mesh.cu, halo.cu).
 r3d_gpu* create_handle(const r3d_params& p, int z0, int nloc, cudaStream_t shared_stream);
 void destroy_handle(r3d_gpu* g);
-void enqueue_step_begin(r3d_gpu* g);
-void enqueue_stage(r3d_gpu* g, int s);  // stage s + BCON; the new state becomes current
+void enqueue_step_begin(r3d_gpu* g, int nstages);
+void enqueue_stage(r3d_gpu* g, int s, int nstages);  // stage s + BCON; the new state becomes current
 void enqueue_step_end(r3d_gpu* g, int nstages);
 // Copies between the device and the caller's arrays, rows of `width` bytes, dense on the host and
 // `pitch` bytes apart on the device, ordered on the handle's stream.  Page-locked host arrays are
@@ -148,6 +151,9 @@ void enqueue_step_end(r3d_gpu* g, int nstages);
 // keeps, the host side by several threads (done when the call returns).
 void to_host(r3d_gpu* g, void* dst, const void* src, size_t pitch, size_t width, size_t rows, const char* what);
 void from_host(r3d_gpu* g, void* dst, const void* src, size_t bytes, const char* what);
+// The tail of a stage launch with the given parts (r3dk::kTail*); plain (flags 0) on a handle whose
+// stages do not take the single-wave form.
+r3dk::StageTail stage_tail(const r3d_gpu* g, int flags);
 // Device pointer and element size of field q of the current state (FP64 or FP32-bulk).
 void* state_field(r3d_gpu* g, int q, size_t* esize);
 int state_fields(const r3d_gpu* g);

@@ -47,7 +47,7 @@ void stage_fp32_box(unsigned* bx, unsigned* by);
 int stage_fp32_ctas_per_sm();
 cudaError_t launch_stage_fp32(int stage, const StageMaps& maps, const Geometry& g, const Physics& ph,
                               const Lines& L, const Background& bg, const FieldSet32& fs, Scalars* sc,
-                              int kchunk, cudaStream_t st);
+                              int kchunk, const StageTail& tail, cudaStream_t st);
 cudaError_t launch_bcon_fp32(const Geometry& g, const Physics& ph, const Lines& L, const Boundary& b,
                              const Background& bg, const FieldSet32& fs, Scalars* sc, int with_dt,
                              cudaStream_t st);
@@ -70,7 +70,9 @@ cudaError_t launch_plane_mean(const Geometry& g, const double* ro, double* rom, 
 void stage_fp64_box(int rows, unsigned* bx, unsigned* by);
 cudaError_t launch_stage_fp64(int stage, const StageMaps& maps, const Geometry& g,
                               const Physics& ph, const Lines& L, const FieldSet& fs, Scalars* sc,
-                              int kchunk, cudaStream_t st, bool emit_rhs = false);
+                              int kchunk, const StageTail& tail, cudaStream_t st, bool emit_rhs = false);
+// whether the FP64 stage has a TAIL form for this configuration (FP32-bulk always has)
+bool stage_fp64_has_tail(const Geometry& g, const Physics& ph);
 cudaError_t launch_bcon(const Geometry& g, const Physics& ph, const Lines& L, const Boundary& b,
                         const FieldSet& fs, Scalars* sc, int with_dt, cudaStream_t st);
 // only_refold: run only if step_end requested a re-evaluation (Scalars::refold)

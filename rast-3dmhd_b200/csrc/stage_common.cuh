@@ -165,7 +165,8 @@ __device__ __forceinline__ void put_periodic(T* f, int64_t base, const Geometry&
 // BCON (src/bcon.cpp:12-141) of one column on the domain's top plane k = 1 (side 0, src/bcon.cpp:
 // 27-98) or bottom plane k = npz (side 1, src/bcon.cpp:104-139), ghost images included; with dt
 // the plane's time-step limits are folded as well.  Bound by latency (its loads all go out first, then
-// two chains of divisions): one thread per column and side, and one copy of the code for both sides.
+// two chains of divisions): one copy of the code serves both sides.  The state is read past L1 (a TAIL
+// stage's other CTAs may have written it).
 __device__ __forceinline__ void bcon_column(const Geometry& g, const Physics& ph, const Lines& L, const Boundary& b,
                                             double* const* x, int side, int i, int j, bool dt, double& m1, double& m2,
                                             double& m3, double& m4, double& mu) {
@@ -219,6 +220,35 @@ __device__ __forceinline__ void bcon_column(const Geometry& g, const Physics& ph
     }
 }
 
+// The sides (bit 0 top, bit 1 bottom) of its column tile whose BCON this CTA runs, decided when the
+// planes kb..ke of its chunk are stored: the plane rewritten and the two inside it lie in one chunk
+// (then its own CTA does it) or in up to three, whose last CTA to arrive does it.  Every thread
+// of the CTA calls it; s is a shared word.
+__device__ __forceinline__ int bcon_sides(const Geometry& g, const StageTail& tail, int kb, int ke, int kchunk,
+                                          bool leader, unsigned int* s) {
+    const bool top = g.top_edge && kb <= 3, bot = g.bot_edge && ke >= g.npz - 2;
+    if (!(tail.flags & kTailBcon) || !(top || bot)) return 0;
+    const int nchunks = (g.npz + kchunk - 1) / kchunk;
+    const unsigned int ntop = min(nchunks, (2 + kchunk) / kchunk), nbot = nchunks - (g.npz - 3) / kchunk;
+    int sides = (top && ntop == 1 ? 1 : 0) | (bot && nbot == 1 ? 2 : 0);
+    const bool ct = top && ntop > 1, cb = bot && nbot > 1;
+    if (ct || cb) {  // uniform over the CTA
+        __threadfence();
+        __syncthreads();
+        if (leader) {
+            unsigned int* cnt = tail.edge_cnt + 2 * (blockIdx.y * gridDim.x + blockIdx.x);
+            unsigned int last = 0;
+            if (ct && atomicInc(cnt, ntop - 1) == ntop - 1) last |= 1;
+            if (cb && atomicInc(cnt + 1, nbot - 1) == nbot - 1) last |= 2;
+            __threadfence();
+            *s = last;
+        }
+        __syncthreads();
+        sides |= (int)*s;
+    }
+    return sides;
+}
+
 // Start of a step (src/step.cpp:133-141, 224-229): dt = sff*min(...).
 __device__ __forceinline__ double step_dt(const Physics& ph, const Scalars* sc) {
     const double w0 = order_value(sc->wmin[0]), w1 = order_value(sc->wmin[1]);
@@ -270,7 +300,7 @@ __device__ __forceinline__ void clear_limits(Scalars* sc) {
 // handle with the threshold filter): the skipped cells have limits > thr_w and a Mach term < thr_um,
 // so the folded limits are exact iff the minima found are <= thr_w and the maximum >= thr_um;
 // otherwise clear them and request the full evaluation (dt_full_kernel with only_refold).  The
-// keys are read past L1: the third stage's other CTAs wrote them.
+// keys are read past L1: a TAIL third stage's other CTAs wrote them.
 __device__ __forceinline__ void step_end(Scalars* sc, int check) {
     sc->nit += 1;
     sc->timc += sc->dt;
@@ -285,6 +315,20 @@ __device__ __forceinline__ void step_end(Scalars* sc, int check) {
         }
     }
     sc->refold = refold;
+}
+
+// True for the CTA that ends the launch: every other CTA of the grid has called this before (and
+// its stores are visible).  Every thread of the CTA calls it; s is a shared word.
+__device__ __forceinline__ bool last_cta(Scalars* sc, bool leader, unsigned int* s) {
+    __syncthreads();
+    if (leader) {
+        const unsigned int n = gridDim.x * gridDim.y * gridDim.z;
+        __threadfence();
+        *s = atomicInc(&sc->ticket, n - 1) == n - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    return *s != 0;
 }
 
 __device__ __forceinline__ uint64_t global_ns() {

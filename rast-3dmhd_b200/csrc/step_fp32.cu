@@ -35,6 +35,7 @@
 #include <cuda_runtime.h>
 
 #include "r3d_kernels.h"
+#include "bcon_fp32.cuh"
 #include "stage_common.cuh"
 #include "tma.cuh"
 
@@ -102,10 +103,11 @@ void stage_fp32_box(unsigned* bx, unsigned* by) {
 }
 int stage_fp32_ctas_per_sm() { return Sh::ctas; }
 
-template <int STAGE>
+// TAIL: the single-wave form (StageTail)
+template <int STAGE, bool TAIL>
 __global__ void __launch_bounds__(Sh::NT, STAGE == 2 ? Sh::ctas_s2 : Sh::ctas)
     stage_fp32(const __grid_constant__ StageMaps maps, Geometry g, Physics ph, Lines L, Background bg,
-               FieldSet32 fs, Scalars* sc, int kchunk) {
+               FieldSet32 fs, Scalars* sc, int kchunk, const __grid_constant__ StageTail tail) {
     constexpr int NT = Sh::NT, RAWF = Sh::RAWF, DERF = Sh::DERF;
     constexpr int RAW_SLOT = Sh::RAW_SLOT, DER_SLOT = Sh::DER_SLOT;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -114,6 +116,8 @@ __global__ void __launch_bounds__(Sh::NT, STAGE == 2 ? Sh::ctas_s2 : Sh::ctas)
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Sh::raw_bytes + Sh::der_bytes);
     __shared__ int s_abort;
     __shared__ DtBounds s_bnd;  // third stage: bounds of the filtered dt fold
+    __shared__ double s_dt;          // TAIL: the step's dt
+    __shared__ unsigned int s_word;  // TAIL
 
     const int tid = threadIdx.x;
     const int ty = tid / PXN, px = tid % PXN;
@@ -166,6 +170,14 @@ __global__ void __launch_bounds__(Sh::NT, STAGE == 2 ? Sh::ctas_s2 : Sh::ctas)
         s_abort = (*(volatile int*)&sc->err != kErrNone) ? 2 : 0;
         tx_extra = sc->tx_extra;
         if (STAGE == 2) s_bnd = sc->bnd;
+        if constexpr (TAIL) {
+            const bool first = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
+            const bool begin = tail.flags & kTailBegin;
+            // the first stage forms dt from the limit keys, which stay until the second clears them
+            s_dt = STAGE == 0 && begin ? step_dt(ph, sc) : sc->dt;
+            if (STAGE == 0 && begin && first) step_begin(ph, sc);
+            if (STAGE == 1 && begin && first) clear_limits(sc);
+        }
         for (int b = 0; b < NRAW; ++b) mbar_init(&bars[b], 1);
         fence_mbar_init();
     }
@@ -181,7 +193,7 @@ __global__ void __launch_bounds__(Sh::NT, STAGE == 2 ? Sh::ctas_s2 : Sh::ctas)
     if (!ok) s_abort = 1;
 
     double m1 = 1e300, m2 = 1e300, m3 = 1e300, m4 = 1e300, mu = 0.0;
-    const double dt = sc->dt;
+    const double dt = TAIL ? s_dt : sc->dt;
     const v2 cg = B2((float)(ph.gam[STAGE] * dt));
     const v2 cz = B2((STAGE < 2) ? (float)(ph.zeta[STAGE + 1] * dt) : 0.0f);
     const int ia = act0 ? i : 1, ib = act1 ? i + 1 : ia, ja = act0 ? j : 1;
@@ -429,28 +441,48 @@ __global__ void __launch_bounds__(Sh::NT, STAGE == 2 ? Sh::ctas_s2 : Sh::ctas)
         }
         return;
     }
+    if constexpr (TAIL) {
+        const int sides = bcon_sides(g, tail, kb, ke, kchunk, tid == 0, &s_word);
+        if (sides) {
+#pragma unroll 1
+            for (int q = 0; q < 4; ++q) {
+                const int side = q >> 1, h = q & 1;
+                if (!(sides >> side & 1) || !(h ? act1 : act0)) continue;
+                bcon_column_fp32(g, ph, L, tail.bnd, bg, fs.xout, side, i + h, j, STAGE == 2, m1, m2, m3, mu);
+            }
+        }
+    }
     if (STAGE == 2) reduce_dt(reinterpret_cast<double*>(der), m1, m2, m3, m4, mu, sc);
+    if constexpr (TAIL && STAGE == 2) {
+        if ((tail.flags & kTailEnd) && last_cta(sc, tid == 0, &s_word) && tid == 0) step_end(sc, 1);
+    }
+}
+
+template <int STAGE, bool TAIL, class... A>
+static void launch_one(dim3 grid, cudaStream_t st, const A&... args) {
+    static bool configured = false;
+    if (!configured) {
+        cudaFuncSetAttribute(stage_fp32<STAGE, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::smem);
+        // all of the unified L1 as shared memory, so that the resident CTAs fit
+        cudaFuncSetAttribute(stage_fp32<STAGE, TAIL>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        configured = true;
+    }
+    stage_fp32<STAGE, TAIL><<<grid, dim3(Sh::NT, 1, 1), Sh::smem, st>>>(args...);
 }
 
 cudaError_t launch_stage_fp32(int stage, const StageMaps& maps, const Geometry& g, const Physics& ph,
                               const Lines& L, const Background& bg, const FieldSet32& fs, Scalars* sc,
-                              int kchunk, cudaStream_t st) {
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(stage_fp32<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::smem);
-        cudaFuncSetAttribute(stage_fp32<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::smem);
-        cudaFuncSetAttribute(stage_fp32<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::smem);
-        // all of the unified L1 as shared memory, so that the resident CTAs fit
-        cudaFuncSetAttribute(stage_fp32<0>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        cudaFuncSetAttribute(stage_fp32<1>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        cudaFuncSetAttribute(stage_fp32<2>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        configured = true;
-    }
-    dim3 block(Sh::NT, 1, 1);
+                              int kchunk, const StageTail& tail, cudaStream_t st) {
     dim3 grid((g.npx + TX - 1) / TX, (g.npy + R3D_F32_TY - 1) / R3D_F32_TY, (g.npz + kchunk - 1) / kchunk);
-    if (stage == 0) stage_fp32<0><<<grid, block, Sh::smem, st>>>(maps, g, ph, L, bg, fs, sc, kchunk);
-    else if (stage == 1) stage_fp32<1><<<grid, block, Sh::smem, st>>>(maps, g, ph, L, bg, fs, sc, kchunk);
-    else stage_fp32<2><<<grid, block, Sh::smem, st>>>(maps, g, ph, L, bg, fs, sc, kchunk);
+    if (tail.flags) {
+        if (stage == 0) launch_one<0, true>(grid, st, maps, g, ph, L, bg, fs, sc, kchunk, tail);
+        else if (stage == 1) launch_one<1, true>(grid, st, maps, g, ph, L, bg, fs, sc, kchunk, tail);
+        else launch_one<2, true>(grid, st, maps, g, ph, L, bg, fs, sc, kchunk, tail);
+    } else {
+        if (stage == 0) launch_one<0, false>(grid, st, maps, g, ph, L, bg, fs, sc, kchunk, tail);
+        else if (stage == 1) launch_one<1, false>(grid, st, maps, g, ph, L, bg, fs, sc, kchunk, tail);
+        else launch_one<2, false>(grid, st, maps, g, ph, L, bg, fs, sc, kchunk, tail);
+    }
     return cudaGetLastError();
 }
 

@@ -154,10 +154,13 @@ void stage_fp64_box(int rows, unsigned* bx, unsigned* by) {
 
 // TF (hydro, itcon 3 only): the top plane's flux is formed as on an interior plane (EdgeTag);
 // IDD (hydro, ID 1 or 2 only): the density diffusion is added to FR (itcon 3 then at run time)
-template <int STAGE, bool KC, bool MHD, bool EMIT, int TYV, bool TF = false, bool IDD = false>
+// TAIL: the stage of a small grid runs BCON and the step's bookkeeping as well (StageTail).  The plain
+// form stays for launches of more than one wave: there the tail hides nothing, and its code cost the
+// main loop 3-8% (504x504x128, FP64 and FP32-bulk) through the registers it keeps.
+template <int STAGE, bool KC, bool MHD, bool EMIT, int TYV, bool TF = false, bool IDD = false, bool TAIL = false>
 __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, TYV>::min_blocks)
     stage_fp64(const __grid_constant__ StageMaps maps, Geometry g, Physics ph, Lines L,
-               FieldSet fs, Scalars* sc, int kchunk) {
+               FieldSet fs, Scalars* sc, int kchunk, const __grid_constant__ StageTail tail) {
     using S = Shape<MHD, TYV>;
     constexpr int NF = S::nf;
     constexpr int TY = S::ty, SN = S::sn, RAWF = S::rawf;
@@ -168,6 +171,8 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::raw_bytes + S::der_bytes);
     __shared__ int s_abort;
     __shared__ DtBounds s_bnd;  // third stage: bounds of the filtered dt fold
+    __shared__ double s_dt;          // TAIL: the step's dt
+    __shared__ unsigned int s_word;  // TAIL
 
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
     const int i0 = 1 + blockIdx.x * TX, j0 = 1 + blockIdx.y * TY;
@@ -243,6 +248,14 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
         s_abort = (*(volatile int*)&sc->err != kErrNone) ? 2 : 0;
         tx_extra = sc->tx_extra;
         if (STAGE == 2) s_bnd = sc->bnd;
+        if constexpr (TAIL) {
+            const bool first = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
+            const bool begin = tail.flags & kTailBegin;
+            // the first stage forms dt from the limit keys, which stay until the second clears them
+            s_dt = STAGE == 0 && begin ? step_dt(ph, sc) : sc->dt;
+            if (STAGE == 0 && begin && first) step_begin(ph, sc);
+            if (STAGE == 1 && begin && first) clear_limits(sc);
+        }
         for (int b = 0; b < NRAW; ++b) mbar_init(&bars[b], 1);
         fence_mbar_init();
     }
@@ -272,7 +285,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
     if (!ok) s_abort = 1;
 
     double m1 = 1e300, m2 = 1e300, m3 = 1e300, m4 = 1e300, mu = 0.0;
-    const double dt = sc->dt;
+    const double dt = TAIL ? s_dt : sc->dt;
     const double cg = ph.gam[STAGE] * dt;
     const double cz = (STAGE < 2) ? ph.zeta[STAGE + 1] * dt : 0.0;
     const double hx = ph.hx, h2x = ph.h2x, hy = ph.hy, hz = ph.hz;
@@ -729,64 +742,91 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
         }
         return;
     }
+    if constexpr (TAIL) {
+        const int sides = bcon_sides(g, tail, kb, ke, kchunk, tid == 0, &s_word);
+        if (sides) {
+#pragma unroll 1
+            for (int q = 0; q < 2 * CPT; ++q) {
+                const int side = q / CPT, j = jr + q % CPT;
+                if (!(sides >> side & 1) || i > g.npx || j > g.npy) continue;
+                bcon_column(g, ph, L, tail.bnd, fs.xout, side, i, j, STAGE == 2, m1, m2, m3, m4, mu);
+            }
+        }
+    }
     if (STAGE == 2 && !EMIT) reduce_dt(der, m1, m2, m3, m4, mu, sc);
+    if constexpr (TAIL && STAGE == 2) {
+        if ((tail.flags & kTailEnd) && last_cta(sc, tid == 0, &s_word) && tid == 0) step_end(sc, 1);
+    }
 }
 
-template <int STAGE, bool KC, bool MHD, bool EMIT, int TYV, bool TF, bool IDD>
+template <int STAGE, bool KC, bool MHD, bool EMIT, int TYV, bool TF, bool IDD, bool TAIL>
 static void launch_one(dim3 grid, const StageMaps& maps, const Geometry& g, const Physics& ph,
-                       const Lines& L, const FieldSet& fs, Scalars* sc, int kchunk, cudaStream_t st) {
+                       const Lines& L, const FieldSet& fs, Scalars* sc, int kchunk, const StageTail& tail,
+                       cudaStream_t st) {
     static bool configured = false;
     constexpr size_t smem = Shape<MHD, TYV>::smem;
+    auto* kernel = stage_fp64<STAGE, KC, MHD, EMIT, TYV, TF, IDD, TAIL>;
     if (!configured) {
-        cudaFuncSetAttribute(stage_fp64<STAGE, KC, MHD, EMIT, TYV, TF, IDD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         // all of the unified L1 as shared memory, so that the resident CTAs fit
-        cudaFuncSetAttribute(stage_fp64<STAGE, KC, MHD, EMIT, TYV, TF, IDD>,
-                             cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         configured = true;
     }
     const dim3 block(TX, TYV / Cells<MHD, STAGE, TYV>::cpt, 1);
-    stage_fp64<STAGE, KC, MHD, EMIT, TYV, TF, IDD><<<grid, block, smem, st>>>(maps, g, ph, L, fs, sc, kchunk);
+    kernel<<<grid, block, smem, st>>>(maps, g, ph, L, fs, sc, kchunk, tail);
 }
 
-template <bool MHD, bool EMIT, int TYV, bool TF = false, bool IDD = false>
+template <bool MHD, bool EMIT, int TYV, bool TF = false, bool IDD = false, bool TAIL = false>
 static void launch_stage(int stage, const StageMaps& maps, const Geometry& g, const Physics& ph,
-                         const Lines& L, const FieldSet& fs, Scalars* sc, int kchunk, cudaStream_t st) {
+                         const Lines& L, const FieldSet& fs, Scalars* sc, int kchunk, const StageTail& tail,
+                         cudaStream_t st) {
     const dim3 grid((g.npx + TX - 1) / TX, (g.npy + TYV - 1) / TYV, (g.npz + kchunk - 1) / kchunk);
-    const bool kc = ph.kappa_const != 0;
-    if (stage == 0) kc ? launch_one<0, true, MHD, EMIT, TYV, TF, IDD>(grid, maps, g, ph, L, fs, sc, kchunk, st)
-                       : launch_one<0, false, MHD, EMIT, TYV, TF, IDD>(grid, maps, g, ph, L, fs, sc, kchunk, st);
-    else if (stage == 1) kc ? launch_one<1, true, MHD, EMIT, TYV, TF, IDD>(grid, maps, g, ph, L, fs, sc, kchunk, st)
-                            : launch_one<1, false, MHD, EMIT, TYV, TF, IDD>(grid, maps, g, ph, L, fs, sc, kchunk, st);
-    else kc ? launch_one<2, true, MHD, EMIT, TYV, TF, IDD>(grid, maps, g, ph, L, fs, sc, kchunk, st)
-            : launch_one<2, false, MHD, EMIT, TYV, TF, IDD>(grid, maps, g, ph, L, fs, sc, kchunk, st);
+    auto launch = [&](auto kc) {
+        constexpr bool KC = decltype(kc)::value;
+        if (stage == 0) launch_one<0, KC, MHD, EMIT, TYV, TF, IDD, TAIL>(grid, maps, g, ph, L, fs, sc, kchunk, tail, st);
+        else if (stage == 1) launch_one<1, KC, MHD, EMIT, TYV, TF, IDD, TAIL>(grid, maps, g, ph, L, fs, sc, kchunk, tail, st);
+        else launch_one<2, KC, MHD, EMIT, TYV, TF, IDD, TAIL>(grid, maps, g, ph, L, fs, sc, kchunk, tail, st);
+    };
+    if (ph.kappa_const) launch(EdgeTag<true>{});
+    else launch(EdgeTag<false>{});
+}
+
+bool stage_fp64_has_tail(const Geometry& g, const Physics& ph) {
+    return g.tile_rows == 8 && (ph.lmag || (!ph.id_mode && !ph.top_free));
 }
 
 template <bool EMIT>
 static void launch_any(int stage, const StageMaps& maps, const Geometry& g, const Physics& ph,
-                       const Lines& L, const FieldSet& fs, Scalars* sc, int kchunk, cudaStream_t st) {
-    if constexpr (!EMIT) {  // ID, itcon 3 (hydro; the adjoint's EMIT recompute refuses them)
+                       const Lines& L, const FieldSet& fs, Scalars* sc, int kchunk, const StageTail& tail,
+                       cudaStream_t st) {
+    if constexpr (!EMIT) {
+        if (tail.flags && stage_fp64_has_tail(g, ph)) {
+            if (ph.lmag) launch_stage<true, false, 8, false, false, true>(stage, maps, g, ph, L, fs, sc, kchunk, tail, st);
+            else launch_stage<false, false, R3D_STAGE_TY, false, false, true>(stage, maps, g, ph, L, fs, sc, kchunk, tail, st);
+            return;
+        }
+        // ID, itcon 3 (hydro; the adjoint's EMIT recompute refuses them)
         if (!ph.lmag && ph.id_mode) {
-            launch_stage<false, false, R3D_STAGE_TY, false, true>(stage, maps, g, ph, L, fs, sc, kchunk, st);
+            launch_stage<false, false, R3D_STAGE_TY, false, true>(stage, maps, g, ph, L, fs, sc, kchunk, tail, st);
             return;
         }
         if (!ph.lmag && ph.top_free) {
-            launch_stage<false, false, R3D_STAGE_TY, true>(stage, maps, g, ph, L, fs, sc, kchunk, st);
+            launch_stage<false, false, R3D_STAGE_TY, true>(stage, maps, g, ph, L, fs, sc, kchunk, tail, st);
             return;
         }
     }
-    if (!ph.lmag) launch_stage<false, EMIT, R3D_STAGE_TY>(stage, maps, g, ph, L, fs, sc, kchunk, st);
-    else if (g.tile_rows == 6) launch_stage<true, EMIT, 6>(stage, maps, g, ph, L, fs, sc, kchunk, st);
-    else launch_stage<true, EMIT, 8>(stage, maps, g, ph, L, fs, sc, kchunk, st);
+    if (!ph.lmag) launch_stage<false, EMIT, R3D_STAGE_TY>(stage, maps, g, ph, L, fs, sc, kchunk, tail, st);
+    else if (g.tile_rows == 6) launch_stage<true, EMIT, 6>(stage, maps, g, ph, L, fs, sc, kchunk, tail, st);
+    else launch_stage<true, EMIT, 8>(stage, maps, g, ph, L, fs, sc, kchunk, tail, st);
 }
 
 cudaError_t launch_stage_fp64(int stage, const StageMaps& maps, const Geometry& g,
                               const Physics& ph, const Lines& L, const FieldSet& fs, Scalars* sc,
-                              int kchunk, cudaStream_t st, bool emit_rhs) {
+                              int kchunk, const StageTail& tail, cudaStream_t st, bool emit_rhs) {
     if (ph.lmag && g.tile_rows != 6 && g.tile_rows != 8) return cudaErrorInvalidValue;
     if (!ph.lmag && g.tile_rows != R3D_STAGE_TY) return cudaErrorInvalidValue;
-    if (emit_rhs) launch_any<true>(stage, maps, g, ph, L, fs, sc, kchunk, st);
-    else launch_any<false>(stage, maps, g, ph, L, fs, sc, kchunk, st);
+    if (emit_rhs) launch_any<true>(stage, maps, g, ph, L, fs, sc, kchunk, tail, st);
+    else launch_any<false>(stage, maps, g, ph, L, fs, sc, kchunk, tail, st);
     return cudaGetLastError();
 }
 
