@@ -622,9 +622,12 @@ void* state_field(r3d_gpu* g, int q, size_t* esize) {
 
 int state_fields(const r3d_gpu* g) { return g->fp32 ? 5 : g->nfields; }
 
-void pull_scalars(r3d_gpu* g, r3d_scalars* sc) {
+void read_scalars(r3d_gpu* g) {  // queued; hsc holds them when the stream has drained
     cuda_ok(cudaMemcpyAsync(g->hsc, g->dsc, sizeof(r3dk::Scalars), cudaMemcpyDeviceToHost, g->stream),
             "scalar read-back");
+}
+
+void take_scalars(r3d_gpu* g, r3d_scalars* sc) {
     cuda_ok(cudaStreamSynchronize(g->stream), "step");
     if (g->hsc->err != r3dk::kErrNone)
         throw Error(R3D_ECUDA, "a stage kernel abandoned a bounded TMA wait (error " +
@@ -642,21 +645,37 @@ void pull_scalars(r3d_gpu* g, r3d_scalars* sc) {
     }
 }
 
-// The graph of two whole steps for the current buffer parity, captured on first use.  Every
-// launch argument of a step is fixed for the handle's lifetime (buffers, TMA maps, physics, the
-// boundary set-up when tc == 0); the step-to-step state lives in device memory.
-cudaGraphExec_t two_step_graph(r3d_gpu* g) {
-    cudaGraphExec_t& ex = g->step_graph[g->cur];
+void pull_scalars(r3d_gpu* g, r3d_scalars* sc) {
+    read_scalars(g);
+    take_scalars(g, sc);
+}
+
+void drop_graphs(r3d_gpu* g) {
+    for (auto* graphs : {g->step_graph, g->single_graph})
+        for (int q = 0; q < 2; ++q) {
+            if (graphs[q]) cudaGraphExecDestroy(graphs[q]);
+            graphs[q] = nullptr;
+        }
+}
+
+// A graph of `steps` whole steps for the current buffer parity (with the read-back of the scalars
+// when read is set), captured on first use.  The launch arguments of a step are fixed between
+// uploads (buffers, TMA maps, physics, the boundary set-up when tc == 0), and an upload that
+// changes them drops the graphs (finish_state); the step-to-step state lives in device memory.
+cudaGraphExec_t captured_steps(r3d_gpu* g, cudaGraphExec_t* slot, int steps, bool read) {
+    cudaGraphExec_t& ex = slot[g->cur];
     if (ex) return ex;
     Range r("r3d.capture");
     const int cur0 = g->cur;
+    g->graph_ph = g->ph;
+    g->graph_bnd = g->bnd;
     Timer off{g, false, nullptr};
     int l = 0, s = 0;
     cuda_ok(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
     cudaGraph_t graph = nullptr;
     try {
-        enqueue_step(g, 3, off, l, s);
-        enqueue_step(g, 3, off, l, s);
+        for (int n = 0; n < steps; ++n) enqueue_step(g, 3, off, l, s);
+        if (read) read_scalars(g);
     } catch (...) {
         cudaStreamEndCapture(g->stream, &graph);
         if (graph) cudaGraphDestroy(graph);
@@ -674,6 +693,10 @@ cudaGraphExec_t two_step_graph(r3d_gpu* g) {
     return ex;
 }
 
+// Steps may be replayed as graphs when nothing about them depends on the host (and one step has
+// gone through the eager path, which configures the kernels).
+bool graph_steps(const r3d_gpu* g) { return g->p.tc == 0.0 && !g->halo; }
+
 void run_steps(r3d_gpu* g, int nsteps, r3d_scalars* sc, r3d_timing* tmout, bool sync) {
     if (!g) throw std::invalid_argument("null handle");
     if (!g->uploaded) throw Error(R3D_ESTATE, "step before upload");
@@ -685,14 +708,14 @@ void run_steps(r3d_gpu* g, int nsteps, r3d_scalars* sc, r3d_timing* tmout, bool 
     // Untimed runs without a host dependency replay a two-step CUDA graph (after one step has
     // gone through the eager path, which configures the kernels): on small grids the nine
     // launches per step would otherwise set the pace.
-    const bool graphs = !tmout && g->p.tc == 0.0 && !g->halo;
+    const bool graphs = !tmout && graph_steps(g);
     if (graphs && g->steps_enqueued == 0 && nsteps > 0) {
         enqueue_step(g, 3, tm, launches, stage_launches);
         ++g->steps_enqueued;
         ++n;
     }
     if (graphs && nsteps - n >= 2) {
-        cudaGraphExec_t ex = two_step_graph(g);
+        cudaGraphExec_t ex = captured_steps(g, g->step_graph, 2, false);
         for (; n + 2 <= nsteps; n += 2) {
             cuda_ok(cudaGraphLaunch(ex, g->stream), "cudaGraphLaunch");
             g->steps_enqueued += 2;
@@ -1044,8 +1067,7 @@ void destroy_handle(r3d_gpu* g) {
     if (!g) return;
     DeviceGuard dg(g->device);
     if (g->stream) cudaStreamSynchronize(g->stream);
-    for (auto& ex : g->step_graph)
-        if (ex) cudaGraphExecDestroy(ex);
+    drop_graphs(g);
     halo_free(g);
     adjoint_free(g);
     cudaFree(g->fscr);
@@ -1193,6 +1215,11 @@ void finish_state(r3d_gpu* g, const r3d_scalars* sc) {
     g->bnd.tb = sc->tb;
     g->host_timc = sc->timc;
     g->host_timi = sc->timi;
+    // a new conductivity profile, metric or bottom temperature: graphs of the old ones are stale
+    if (std::memcmp(&g->graph_ph, &g->ph, sizeof g->ph) || std::memcmp(&g->graph_bnd, &g->bnd, sizeof g->bnd)) {
+        cuda_ok(cudaStreamSynchronize(g->stream), "upload");  // none of them is running
+        drop_graphs(g);
+    }
     // counters that an abandoned stage may have left mid-way start over
     if (g->tail) cuda_ok(cudaMemsetAsync(g->edge_cnt, 0, g->edge_bytes, g->stream), "reset");
     cuda_ok(r3dk::launch_reset_reduction(g->dsc, g->stream), "reset");
@@ -1498,11 +1525,23 @@ int r3d_gpu_step(r3d_gpu* g, int nstages, r3d_scalars* sc) {
         if (nstages < 1 || nstages > 3) throw std::invalid_argument("nstages must be 1..3");
         if (!g->uploaded) throw Error(R3D_ESTATE, "step before upload");
         DeviceGuard dg(g->device);
-        Timer tm{g, false, nullptr};
-        int a = 0, b = 0;
-        enqueue_step(g, nstages, tm, a, b);
         r3d_scalars tmp{};
-        pull_scalars(g, &tmp);
+        if (nstages == 3 && g->steps_enqueued > 0 && graph_steps(g)) {
+            // one launch for the step and its read-back: at 32x32x64 the eager launches and the copy
+            // took 42 us per step beside 42 us of kernels
+            cudaGraphExec_t ex = captured_steps(g, g->single_graph, 1, true);
+            cuda_ok(cudaGraphLaunch(ex, g->stream), "cudaGraphLaunch");
+            g->cur = 1 - g->cur;  // three stages
+            g->work_ok = true;
+            ++g->steps_enqueued;
+            take_scalars(g, &tmp);
+        } else {
+            Timer tm{g, false, nullptr};
+            int a = 0, b = 0;
+            enqueue_step(g, nstages, tm, a, b);
+            if (nstages == 3) ++g->steps_enqueued;
+            pull_scalars(g, &tmp);
+        }
         if (sc) *sc = tmp;
         if (!std::isfinite(tmp.dt)) throw Error(R3D_ENUMERIC, "non-finite dt");
     });

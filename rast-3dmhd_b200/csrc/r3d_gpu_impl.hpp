@@ -69,6 +69,10 @@ struct r3d_gpu {
     // two whole steps captured as a CUDA graph, one per state-buffer parity at capture (r3d_gpu_run
     // replays it; six stages leave the parity unchanged)
     cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
+    // one whole step and the read-back of its scalars, per parity (r3d_gpu_step)
+    cudaGraphExec_t single_graph[2] = {nullptr, nullptr};
+    r3dk::Physics graph_ph{};   // the arguments the graphs were captured with that an upload may change
+    r3dk::Boundary graph_bnd{};
     int64_t steps_enqueued = 0;
     void* bounce[2] = {nullptr, nullptr};  // page-locked copy buffers (to_host, from_host)
     cudaEvent_t bounce_ev[2] = {nullptr, nullptr};
