@@ -18,8 +18,8 @@
 // streams the state fields of each plane, with a one-cell x/y halo, into a ring by TMA (one
 // (34, TY+2, 1) box per field, completion on a per-slot mbarrier), two planes ahead of the
 // plane being computed.  Each loaded cell is then turned once into u, v, w (and, with MHD,
-// 1/rho and P = rho*T; src/fluxes.cpp:131-166) in a second, 4-slot ring, so a single
-// __syncthreads per plane orders everything: the plane k+1 derivation, the TMA refill of the
+// 1/rho and P = rho*T; src/fluxes.cpp:131-166) in a second, 4-slot ring, so a single barrier
+// per plane (__syncthreads; MHD: an mbarrier) orders everything: the plane k+1 derivation, the TMA refill of the
 // slot of plane k-2 (hydro: of plane k-1, whose values the threads hold), and the compute of
 // plane k, which reads the 19-point stencil (the twelve edge neighbours of u, v, w come from
 // the cross terms :367-374, :449-456, :496-498) from shared memory.  Hydro threads compute two
@@ -181,6 +181,12 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
     const int i = i0 + tx, jr = j0 + ty * CPT;  // the thread's column and first row
 
     constexpr bool LEAN = Ring<MHD>::lean;
+    // MHD: the plane barrier in two halves.  A warp arrives when it has derived its part of plane k+1
+    // and waits only before it first reads planes k+1 and k-1, after the velocity differences within
+    // plane k: with two CTAs per SM a whole barrier cost 0.9 of 6 cycles per issue (126x126x256 on
+    // B200, per step: 829 -> 818 us; with the field differences ahead of the wait too, which spills,
+    // 860).  Hydro (three CTAs per SM) was 1.5% slower with it, the FP32-bulk stage 11%.
+    constexpr bool SPLIT = MHD;
     // hydro: rows of the thread whose accumulators are loaded before the fluxes, the others after
     constexpr int ZE = (LEAN && STAGE > 0 && CPT > 1) ? 1 : 0;
     constexpr int NRAW = Ring<MHD>::nraw;
@@ -257,6 +263,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
             if (STAGE == 1 && begin && first) clear_limits(sc);
         }
         for (int b = 0; b < NRAW; ++b) mbar_init(&bars[b], 1);
+        if (SPLIT) mbar_init(&bars[NRAW], NTH / 32);
         fence_mbar_init();
     }
     __syncthreads();
@@ -311,6 +318,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
         }
     }
 
+    if (SPLIT) __syncthreads();  // planes kb-1 and kb derived
     for (int k = kb; k <= ke; ++k) {
         const int q = k - (kb - 1);
         // the RK accumulators Z of the thread's cells: the next plane's into L2, this plane's
@@ -342,12 +350,22 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
         };
         if constexpr (!LEAN) load_z(0, CPT);  // MHD: issued before the derive phase and the barrier
         if (!derive(k + 1)) s_abort = 1;
-        __syncthreads();
-        if (s_abort) break;
-        if (tid == 0 && k + 2 <= ke + 1) {
-            fence_proxy_async();
-            issue(k + 2);
+        if constexpr (SPLIT) {
+            __syncwarp();
+            if (tx == 0) mbar_arrive(&bars[NRAW]);
+        } else {
+            __syncthreads();
+            if (s_abort) break;
         }
+        // plane k+1 is derived and the slot of plane k+2 is free
+        auto plane_ready = [&] {
+            if (SPLIT && !mbar_wait(&bars[NRAW], (k - kb) & 1)) s_abort = 1;
+            if (tid == 0 && k + 2 <= ke + 1 && !(SPLIT && s_abort)) {
+                fence_proxy_async();
+                issue(k + 2);
+            }
+        };
+        if constexpr (!SPLIT) plane_ready();
         const double* rm = raw + ((q + NRAW - 1) % NRAW) * S::raw_slot;
         const double* r0 = raw + (q % NRAW) * S::raw_slot;
         const double* rp = raw + ((q + 1) % NRAW) * S::raw_slot;
@@ -385,6 +403,24 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
             // ---- continuity, src/fluxes.cpp:87-121 ----
             double fr = (RW_(r0, R_RU, -1, 0) - RW_(r0, R_RU, 1, 0)) * hx * dx1;
             fr -= (RW_(r0, R_RV, 0, 1) - RW_(r0, R_RV, 0, -1)) * tmpy;
+            const double U0 = DV_(d0, D_U, 0, 0), V0 = DV_(d0, D_V, 0, 0), W0 = DV_(d0, D_W, 0, 0);
+            const double ri = LEAN ? riq[c] : DV_(d0, D_RI, 0, 0);
+            const double Uxp = DV_(d0, D_U, 1, 0), Uxm = DV_(d0, D_U, -1, 0);
+            const double Uyp = DV_(d0, D_U, 0, 1), Uym = DV_(d0, D_U, 0, -1);
+            const double Vxp = DV_(d0, D_V, 1, 0), Vxm = DV_(d0, D_V, -1, 0);
+            const double Vyp = DV_(d0, D_V, 0, 1), Vym = DV_(d0, D_V, 0, -1);
+            const double Wxp = DV_(d0, D_W, 1, 0), Wxm = DV_(d0, D_W, -1, 0);
+            const double Wyp = DV_(d0, D_W, 0, 1), Wym = DV_(d0, D_W, 0, -1);
+            // velocity gradients, the reference's WW1..WW3 / RU..RW temporaries
+            const double ux = (Uxp - Uxm) * hx * dx1;  // src/fluxes.cpp:331,416; 3dmhdsub.f:2151
+            const double vx = (Vxp - Vxm) * hx * dx1;  // :336; 3dmhdsub.f:2157
+            const double wx = (Wxp - Wxm) * hx * dx1;  // :341,505; 3dmhdsub.f:2163
+            const double uy = (Uyp - Uym) * hy * dyj;  // :382; 3dmhdsub.f:2181
+            const double vy = (Vyp - Vym) * hy * dyj;  // :397; 3dmhdsub.f:2187
+            const double wy = (Wyp - Wym) * hy * dyj;  // :476; 3dmhdsub.f:2193
+            if constexpr (SPLIT) {
+                if (c == 0) plane_ready();
+            }
             double dwz;
             if (EDGE && k == 1 && g.top_edge)
                 dwz = (4.0 * RW_(rp, R_RW, 0, 0) - fs.xin[R_RW][nc + 2 * PL]) * tmpz;
@@ -418,24 +454,9 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
             double fu = 0.0, fv = 0.0, fw = 0.0, ft = 0.0;
             double b1 = 0.0, b2f = 0.0, b3 = 0.0;  // B fluxes WW1..WW3 (MHD)
             const double dzk = L.dzzdz[k];
-            const double U0 = DV_(d0, D_U, 0, 0), V0 = DV_(d0, D_V, 0, 0), W0 = DV_(d0, D_W, 0, 0);
-            const double ri = LEAN ? riq[c] : DV_(d0, D_RI, 0, 0);
-            const double Uxp = DV_(d0, D_U, 1, 0), Uxm = DV_(d0, D_U, -1, 0);
-            const double Uyp = DV_(d0, D_U, 0, 1), Uym = DV_(d0, D_U, 0, -1);
             const double Uzp = DV_(dp, D_U, 0, 0), Uzm = DV_(dm, D_U, 0, 0);
-            const double Vxp = DV_(d0, D_V, 1, 0), Vxm = DV_(d0, D_V, -1, 0);
-            const double Vyp = DV_(d0, D_V, 0, 1), Vym = DV_(d0, D_V, 0, -1);
             const double Vzp = DV_(dp, D_V, 0, 0), Vzm = DV_(dm, D_V, 0, 0);
-            const double Wxp = DV_(d0, D_W, 1, 0), Wxm = DV_(d0, D_W, -1, 0);
-            const double Wyp = DV_(d0, D_W, 0, 1), Wym = DV_(d0, D_W, 0, -1);
             const double Wzp = DV_(dp, D_W, 0, 0), Wzm = DV_(dm, D_W, 0, 0);
-            // velocity gradients, the reference's WW1..WW3 / RU..RW temporaries
-            const double ux = (Uxp - Uxm) * hx * dx1;  // src/fluxes.cpp:331,416; 3dmhdsub.f:2151
-            const double vx = (Vxp - Vxm) * hx * dx1;  // :336; 3dmhdsub.f:2157
-            const double wx = (Wxp - Wxm) * hx * dx1;  // :341,505; 3dmhdsub.f:2163
-            const double uy = (Uyp - Uym) * hy * dyj;  // :382; 3dmhdsub.f:2181
-            const double vy = (Vyp - Vym) * hy * dyj;  // :397; 3dmhdsub.f:2187
-            const double wy = (Wyp - Wym) * hy * dyj;  // :476; 3dmhdsub.f:2193
             const double uz = (Uzp - Uzm) * hz * dzk;  // :464; 3dmhdsub.f:2211
             const double vz = (Vzp - Vzm) * hz * dzk;  // :469; 3dmhdsub.f:2217
             const double wz = (Wzp - Wzm) * hz * dzk;  // :423; 3dmhdsub.f:2223
@@ -667,6 +688,7 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
                 rhs(EdgeTag<true>{});
             }
         }
+        if (SPLIT && s_abort) break;
         if constexpr (LEAN) {
             // hydro: the other rows' accumulators (prefetched into L2 a plane earlier), loaded after
             // the fluxes; the compiler barrier keeps the loads from being hoisted into them
