@@ -404,10 +404,11 @@ struct Fp64Staging {
     unsigned blocks() const { return (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16); }
 };
 
-// The bounce buffers: 8 MB each, small enough to stay cheap and large enough that a chunk's device
-// copy (0.16 ms) hides its launch.  Measured on B200, 16 host cores, pageable numpy arrays: 128x128x128
-// adjoint_step 27.2 ms with the driver's own staging of pageable copies.
-constexpr size_t kBounce = size_t(8) << 20, kDirect = size_t(1) << 19;
+// The bounce buffers: 8 MB each, large enough that a chunk's device copy hides behind the host's (2 MB
+// chunks were 10% slower).  Page-locking costs about 1 ms per MB once per handle, so arrays below 4 MB
+// stay with the driver's own staging: there a first call would pay more than it saves.  B200, 16 host
+// cores: 128x128x128 adjoint_step (17.6 MB per field each way) 27.2 ms with the driver's staging, 12.6.
+constexpr size_t kBounce = size_t(8) << 20, kDirect = size_t(4) << 20;
 
 bool pageable(const void* p) {
     cudaPointerAttributes at{};

@@ -4,8 +4,8 @@
   in one, two or three chunks; larger launches cut the planned chunks: bit for bit the oracle's.
 * The reverse sweep's BCON transpose takes one side per thread from npz = 6 on, both in turn below;
   its tiles are 32 x 8: dot products against the exact tangent.
-* Host arrays are copied directly when page-locked or small and through page-locked buffers in 8 MB
-  chunks when pageable: the same arrays either way.
+* Host arrays are copied directly when page-locked or below 4 MB and through page-locked buffers in
+  8 MB chunks when pageable: the same arrays either way.
 """
 import numpy as np
 import pytest
@@ -89,8 +89,8 @@ def test_adjoint_step_dot_product(flags):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape", [(20, 20, 30), (64, 50, 40), (64, 64, 300)],
-                         ids=["direct", "one_chunk", "chunks"])  # 0.12, 1.1 and 10.5 MB per field
+@pytest.mark.parametrize("shape", [(20, 20, 30), (64, 64, 120), (64, 64, 300)],
+                         ids=["direct", "one_chunk", "chunks"])  # 0.12, 4.3 and 10.5 MB per field
 @pytest.mark.parametrize("precision", ["fp64", "fp32bulk"])
 def test_pageable_and_page_locked_arrays(shape, precision):
     import torch
