@@ -28,6 +28,7 @@
 #include "adjoint_cell.cuh"
 #include "r3d_gpu_impl.hpp"
 #include "stage_common.cuh"
+#include "tma.cuh"
 
 using namespace r3db;
 using r3dk::AdjArgs;
@@ -35,6 +36,7 @@ using r3dk::AdjArgs;
 namespace {
 
 constexpr int BX = 32, BY = 8;       // cells per block of the passes
+constexpr int kPassBlocks = 2;      // blocks of pass 2 resident per SM
 constexpr int kDotBlocks = 32;        // partial sums of the dt dot products
 
 struct AdjScalars {
@@ -80,7 +82,7 @@ __global__ void __launch_bounds__(BX* BY) adj_bcon_kernel(r3dk::Geometry g, r3dk
 
 // Bound by the latency of the gathers, so by how many loads the warps of an SM keep in flight: two
 // 256-thread blocks per SM (three for hydro pass 1) with every load of a cell free to go out at once.
-// B200, us per stage: 128x128x128 hydro pass 1 154 (two blocks: 165), pass 2 170 (three blocks, 80
+// B200, us per stage: 128x128x128 hydro pass 1 154 (two blocks: 165), pass 2 170 without its prefetch (three blocks, 80
 // registers and spills: 192); 64x64x128 MHD pass 1 69 (three: 77), pass 2 87 (three: 97).  The passes
 // they replace, which stored every Lambda and folded lambda_F separately: 577 and 222.
 template <bool MHD>
@@ -93,8 +95,30 @@ __global__ void __launch_bounds__(BX* BY, MHD ? 2 : 3) adj_pass1_kernel(const __
     block_sum_store(dot, dots);
 }
 
+// The cell of this thread in the block `ahead` places later in launch order (-1: none): with as many
+// places as blocks run at once, its lines are in L2 by the time that block gathers them (pass 2,
+// 128x128x128 hydro 170 -> 143 us, 64x64x128 MHD 87 -> 84; twice as far ahead 151 and 96.  Pass 1, whose
+// gathers are fewer, was 5% slower with it).
+__device__ __forceinline__ int cell_ahead(const r3dk::Geometry& g, int ahead) {
+    const int b = block_linear() + ahead, row = b / (int)gridDim.x;
+    const int i = 1 + (b % (int)gridDim.x) * BX + threadIdx.x;
+    const int j = 1 + (row % (int)gridDim.y) * BY + threadIdx.y, k = 1 + row / (int)gridDim.y;
+    if (i > g.npx || j > g.npy || k > g.npz) return -1;
+    return k * (int)g.plane + j * (int)g.pitch + i;
+}
+
 template <bool MHD>
 __global__ void __launch_bounds__(BX* BY, 2) adj_pass2_kernel(const __grid_constant__ AdjArgs A) {
+    if (const int n = cell_ahead(A.g, A.ahead); n >= 0) {
+#pragma unroll
+        for (int f = 0; f < (MHD ? 8 : 5); ++f) {
+            r3dk::prefetch_l2(A.x + f * A.fe + n);
+            r3dk::prefetch_l2(A.a + f * A.fe + n);
+            r3dk::prefetch_l2(A.out + f * A.fe + n);
+        }
+#pragma unroll
+        for (int q = 0; q < (MHD ? r3dk::kMidMax : r3dk::kMidHydro); ++q) r3dk::prefetch_l2(A.mid + q * A.fe + n);
+    }
     const int i = 1 + blockIdx.x * BX + threadIdx.x;
     const int j = 1 + blockIdx.y * BY + threadIdx.y;
     const int k = 1 + blockIdx.z;
@@ -378,6 +402,7 @@ void reverse_step(r3d_gpu* g, Adjoint* A, const double* src) {
         p.out = other;
         p.F = A->F[s];
         p.sc = A->asc;
+        p.ahead = g->num_sms * kPassBlocks;
         p.gam = g->ph.gam[s];
         p.zeta = s < 2 ? g->ph.zeta[s + 1] : 0.0;
         double* dots = A->dots + (size_t)s * A->nblocks;

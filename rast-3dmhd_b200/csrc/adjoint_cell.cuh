@@ -75,6 +75,7 @@ struct AdjArgs {
     const double* F;      // F(X_s), for d/d(dt)
     const Scalars* sc;    // dt of the step
     double gam, zeta;     // gam_s, zeta_{s+1}
+    int ahead;            // blocks by which the L2 prefetch runs ahead
 };
 
 struct Nbr {  // neighbour offsets of an interior cell on the x/y torus
