@@ -82,9 +82,10 @@ __global__ void __launch_bounds__(BX* BY) adj_bcon_kernel(r3dk::Geometry g, r3dk
 
 // Bound by the latency of the gathers, so by how many loads the warps of an SM keep in flight: two
 // 256-thread blocks per SM (three for hydro pass 1) with every load of a cell free to go out at once.
-// B200, us per stage: 128x128x128 hydro pass 1 154 (two blocks: 165), pass 2 170 without its prefetch (three blocks, 80
-// registers and spills: 192); 64x64x128 MHD pass 1 69 (three: 77), pass 2 87 (three: 97).  The passes
-// they replace, which stored every Lambda and folded lambda_F separately: 577 and 222.
+// B200, us per stage, while lambda_Y was still added by pass 1 and pass 2 did not prefetch:
+// 128x128x128 hydro pass 1 154 (two blocks: 165), pass 2 170 (three blocks, 80 registers and spills:
+// 192); 64x64x128 MHD pass 1 69 (three: 77), pass 2 87 (three: 97).  Now 150 + 152 and 65 + 95.  The
+// passes they replace, which stored every Lambda and folded lambda_F separately: 577 and 222.
 template <bool MHD>
 __global__ void __launch_bounds__(BX* BY, MHD ? 2 : 3) adj_pass1_kernel(const __grid_constant__ AdjArgs A, double* dots) {
     const int i = 1 + blockIdx.x * BX + threadIdx.x;
@@ -97,8 +98,8 @@ __global__ void __launch_bounds__(BX* BY, MHD ? 2 : 3) adj_pass1_kernel(const __
 
 // The cell of this thread in the block `ahead` places later in launch order (-1: none): with as many
 // places as blocks run at once, its lines are in L2 by the time that block gathers them (pass 2,
-// 128x128x128 hydro 170 -> 143 us, 64x64x128 MHD 87 -> 84; twice as far ahead 151 and 96.  Pass 1, whose
-// gathers are fewer, was 5% slower with it).
+// 128x128x128 hydro 170 -> 143 us, 64x64x128 MHD 87 -> 84, both before it also read lambda_Y; twice as
+// far ahead 151 and 96.  Pass 1, whose gathers are fewer, was 5% slower with it).
 __device__ __forceinline__ int cell_ahead(const r3dk::Geometry& g, int ahead) {
     const int b = block_linear() + ahead, row = b / (int)gridDim.x;
     const int i = 1 + (b % (int)gridDim.x) * BX + threadIdx.x;
@@ -115,6 +116,7 @@ __global__ void __launch_bounds__(BX* BY, 2) adj_pass2_kernel(const __grid_const
             r3dk::prefetch_l2(A.x + f * A.fe + n);
             r3dk::prefetch_l2(A.a + f * A.fe + n);
             r3dk::prefetch_l2(A.out + f * A.fe + n);
+            r3dk::prefetch_l2(A.lam + f * A.fe + n);
         }
 #pragma unroll
         for (int q = 0; q < (MHD ? r3dk::kMidMax : r3dk::kMidHydro); ++q) r3dk::prefetch_l2(A.mid + q * A.fe + n);

@@ -15,15 +15,16 @@
 //     depends on du/dy + dv/dx (and its two companions) as a whole, and the Lorentz force and
 //     ohmic heating on the curl, so six arrays (nine with MHD) carry what the heating, the p dV
 //     work and the current contribute.  The partials w.r.t. u, v, w, 1/rho, T, B at c itself go
-//     through the chain rule here (u = RU/rho, P = rho*T, 1/rho) and wait, with lambda_Y, in the
-//     output array.
+//     through the chain rule here (u = RU/rho, P = rho*T, 1/rho) and wait in the output array.
 //   pass 2 (per input cell m): adds the transposed difference stencils, gathered at the neighbours
 //     of m (a central difference coef(c)*(f(c+e) - f(c-e)) contributes coef(m-e)*Lambda(m-e) -
 //     coef(m+e)*Lambda(m+e) to f's adjoint at m).  Every Lambda not stored is a product of values
 //     at one point - lambda_F times u, v, w, 1/rho, B - and is formed where it is gathered; the
-//     cross differences of the viscous stress are corner stencils of lambda_F itself.
+//     cross differences of the viscous stress are corner stencils of lambda_F itself.  lambda_Y, the
+//     largest term, is added last: added in pass 1 it was rounded again with every term that followed
+//     (128x128x128 hydro vjp, error against 64-bit torch 1.4e-16; 2.9e-17 so).
 //
-// Bound: the latency of the gathers, then DRAM.  One stage moves 98 arrays (MHD) where the form that
+// Bound: the latency of the gathers, then DRAM.  One stage moves 106 arrays (MHD) where the form that
 // stored all 33 Lambda arrays and folded lambda_F in a pass of its own moved 146; splitting the
 // partials off pass 2 keeps it at 128 registers (with them it needed 174 and ran at 8 warps
 // per SM: 200 us at 64x64x128 MHD against 87).
@@ -151,8 +152,8 @@ R3D_HD double adj_pass1_cell(const AdjArgs& A, int i, int j, int k) {
     for (int f = 0; f < NF; ++f) a[f] = A.lprev ? A.lprev[f * fe + n] : 0.0;
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
-        own[f] = lam[f * fe + n];  // the Z path
-        a[f] = cg * own[f] + cz * a[f];
+        own[f] = 0.0;
+        a[f] = cg * lam[f * fe + n] + cz * a[f];
         dot += F[f * fe + n] * a[f];
     }
 #pragma unroll
@@ -239,7 +240,7 @@ R3D_HD void adj_pass2_cell(const AdjArgs& A, int i, int j, int k) {
     const int n = b.n, zp = n + PL, zm = n - PL;
     const bool lo = k > 1, hi = k < npz;
     const int64_t fe = A.fe;
-    const In x{A.x}, a{A.a}, md{A.mid};
+    const In x{A.x}, a{A.a}, md{A.mid}, lam{A.lam};
     const In mu = x.field(F_RU * fe), mv = x.field(F_RV * fe), mw = x.field(F_RW * fe), ro = x.field(F_RO * fe);
     const In aU = a.field(F_RU * fe), aV = a.field(F_RV * fe), aW = a.field(F_RW * fe), aR = a.field(F_RO * fe);
     const In aT = a.field(F_TT * fe);
@@ -395,7 +396,7 @@ R3D_HD void adj_pass2_cell(const AdjArgs& A, int i, int j, int k) {
         own[F_BZ] += lB3;
     }
 #pragma unroll
-    for (int f = 0; f < NF; ++f) A.out[f * fe + n] = own[f];
+    for (int f = 0; f < NF; ++f) A.out[f * fe + n] = own[f] + lam[f * fe + n];  // the Z path
 }
 
 // ------------------------------------------------------------------- BCON^T -------------
