@@ -181,7 +181,8 @@ __global__ void adj_dt_apply_kernel(r3dk::Geometry g, r3dk::Physics ph, r3dk::Li
     const unsigned long long an = aux->argmin;
     double mstar;
     const int term = r3dk::winning_limit(aux->wkey, ph.lmag, mstar);
-    if (term == 3 || an == ~0ull) return;
+    // sff == 0: dt is 0 whatever the state (and nothing to divide the sums by)
+    if (term == 3 || an == ~0ull || ph.sff == 0.0) return;
     double lam_dt = 0.0;
     for (int b = 0; b < kDotBlocks; ++b) lam_dt += aux->part[b];
     lam_dt /= sc->dt;
