@@ -229,6 +229,8 @@ struct Adjoint {
     double* dots = nullptr;
     int nblocks = 0;
     r3dk::Scalars* asc = nullptr;   // scalars of the recompute
+    unsigned int* edge_cnt = nullptr;  // the recompute's own BCON counters: a stage it abandons leaves the
+                                       // forward steps' ones alone
     AdjScalars* aux = nullptr;
     AdjScalars* haux = nullptr;     // pinned mirror
     std::vector<double*> ckpt;      // recorded checkpoints
@@ -281,9 +283,11 @@ Adjoint* workspace(r3d_gpu* g) {
         A->nblocks = (int)(gr.x * gr.y * gr.z);
         A->dots = dalloc(A, (size_t)3 * A->nblocks);
         cuda_ok(cudaMalloc(&A->asc, sizeof(r3dk::Scalars)), "cudaMalloc(adjoint scalars)");
-        cuda_ok(cudaMemsetAsync(A->asc, 0, sizeof(r3dk::Scalars), g->stream), "cudaMemset");
+        if (g->tail) {
+            cuda_ok(cudaMalloc(&A->edge_cnt, g->edge_bytes), "cudaMalloc(counters)");
+            A->bytes += (int64_t)g->edge_bytes;
+        }
         cuda_ok(cudaMalloc(&A->aux, sizeof(AdjScalars)), "cudaMalloc(adjoint scalars)");
-        cuda_ok(cudaMemsetAsync(A->aux, 0, sizeof(AdjScalars), g->stream), "cudaMemset");
         cuda_ok(cudaMallocHost(&A->haux, sizeof(AdjScalars)), "cudaMallocHost");
         // the z ghost planes of a and mid are read (with weight 0) and stay zero; keep every
         // other buffer defined as well
@@ -356,6 +360,17 @@ r3dk::StageMaps state_maps(const r3d_gpu* g, const Adjoint* A, const double* bas
     return m;
 }
 
+// Start of a sweep: nothing an earlier one left (an error flag, counters of a stage that was abandoned
+// mid-way, differing values) counts in this one.
+void begin_sweep(r3d_gpu* g, Adjoint* A) {
+    cuda_ok(cudaMemsetAsync(A->asc, 0, sizeof(r3dk::Scalars), g->stream), "cudaMemset");
+    cuda_ok(cudaMemcpyAsync(&A->asc->tx_extra, &g->dsc->tx_extra, sizeof(g->dsc->tx_extra), cudaMemcpyDeviceToDevice,
+                            g->stream),
+            "tx_extra");
+    cuda_ok(cudaMemsetAsync(A->aux, 0, sizeof(AdjScalars), g->stream), "cudaMemset");
+    if (A->edge_cnt) cuda_ok(cudaMemsetAsync(A->edge_cnt, 0, g->edge_bytes, g->stream), "cudaMemset");
+}
+
 // One forward step from the state src with the dt of the limit minima key, through S[1] and S[2]
 // into dst; emit: F[0..2] stored.
 void recompute_step(r3d_gpu* g, Adjoint* A, const unsigned long long* key, const double* src, double* dst, bool emit) {
@@ -366,7 +381,8 @@ void recompute_step(r3d_gpu* g, Adjoint* A, const unsigned long long* key, const
     for (int s = 0; s < 3; ++s) {
         r3dk::FieldSet fs = stage_fields(A, s, in[s], out[s]);
         // (the EMIT stages have no single-wave form)
-        const r3dk::StageTail tail = emit ? r3dk::StageTail{} : stage_tail(g, r3dk::kTailBcon);
+        r3dk::StageTail tail = emit ? r3dk::StageTail{} : stage_tail(g, r3dk::kTailBcon);
+        tail.edge_cnt = A->edge_cnt;
         cuda_ok(r3dk::launch_stage_fp64(s, state_maps(g, A, in[s]), g->geo, g->ph, g->lines, fs, A->asc, g->depth, tail,
                                         g->stream, emit),
                 "adjoint recompute stage");
@@ -487,6 +503,7 @@ void adjoint_free(r3d_gpu* g) {
     cudaFree(A->mid);
     cudaFree(A->dots);
     cudaFree(A->asc);
+    cudaFree(A->edge_cnt);
     cudaFree(A->aux);
     if (A->haux) cudaFreeHost(A->haux);
     impl::free_states(A->ckpt);
@@ -550,7 +567,7 @@ int r3d_gpu_adjoint_backward(r3d_gpu* g, const double* const* seed, double* cons
         resize_states(A, A->seg, std::min(K, N) - 1);
         for (int s = 1; s < 4; ++s) copy_ghost_planes(g, A, A->S[s], A->ckpt[0]);
         for (double* p : A->seg) copy_ghost_planes(g, A, p, A->ckpt[0]);
-        cuda_ok(cudaMemsetAsync(&A->aux->mismatch, 0, sizeof(unsigned long long), g->stream), "cudaMemset");
+        begin_sweep(g, A);
         upload_seed(g, A, seed);
         const double* final_state = A->ckpt.back();  // the recorded final state
         {
@@ -582,6 +599,7 @@ int r3d_gpu_adjoint_step(r3d_gpu* g, const double* const* seed, double* const* g
         if (!A->S[0]) A->S[0] = dalloc(A, (size_t)A->nf * A->field_elems);
         save_current(g, A, A->S[0]);
         for (int s = 1; s < 4; ++s) copy_ghost_planes(g, A, A->S[s], A->S[0]);
+        begin_sweep(g, A);
         upload_seed(g, A, seed);
         cuda_ok(r3dk::launch_reset_reduction(A->asc, g->stream), "adjoint reset");
         cuda_ok(r3dk::launch_dt_full(g->geo, g->ph, g->lines, stage_fields(A, 0, A->S[0], A->S[1]), A->asc, g->stream),

@@ -43,3 +43,61 @@ def test_zero_safety_factor(extra):
         # each, every one rounded: 30 eps of the summed sizes a step
         size = sum(float(np.abs(t).sum()) for t in left + right)
         assert abs(lhs - rhs) <= 30 * steps * 2.0 ** -53 * size, (lhs, rhs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("extra", [["--npx", "32", "--npy", "32", "--npz", "64"]], ids=["hydro"])
+def test_abandoned_recompute_leaves_nothing_behind(extra):
+    """The recompute's bounded waits run out (single-wave stages, BCON planes in several chunks for hydro): the
+    sweep reports it, and the forward steps, the sweeps and the trajectory after it are as without it."""
+    p = R.parse(extra + ["--seed", "3"])
+    st = R.HostState.setup(p)
+    rng = np.random.default_rng(2)
+    lam = {n: rng.standard_normal(a.shape) for n, a in st.fields.items()}
+
+    def session(fail):
+        out = []
+        with R.GpuSim(p) as sim:
+            sim.upload(st)
+            sim.adjoint_record(4, 3)
+            for call in (sim.adjoint_backward, sim.adjoint_step) if fail else ():
+                sim.debug_tma_extra(16)
+                with pytest.raises(R.R3dError) as e:
+                    call(lam)
+                assert e.value.code == R.R3D_ECUDA and "bounded TMA wait" in str(e.value)
+                sim.debug_tma_extra(0)
+            dts = [sim.step()["dt"] for _ in range(3)]
+            got = st.copy()
+            sim.download(got)
+            out = [got.fields, sim.adjoint_step(lam), sim.adjoint_backward(lam)]
+        return dts, out
+
+    ref, got = session(False), session(True)
+    assert got[0] == ref[0]
+    for a, b in zip(got[1], ref[1]):
+        for n in a:
+            assert np.array_equal(a[n], b[n]), n
+
+
+@pytest.mark.gpu
+def test_diverged_recompute_is_reported_once():
+    """A recompute that differs from the recorded trajectory (here: another conductivity profile uploaded in
+    between) is an error of that sweep, not of the next."""
+    p = R.parse(["--npx", "24", "--npy", "20", "--npz", "36", "--seed", "3"])
+    st = R.HostState.setup(p)
+    other = st.copy()
+    other.lines["rkapa"] = 1.0 + 0.1 * np.linspace(0.0, 1.0, p.npz + 2)
+    lam = {n: np.ones_like(a) for n, a in st.fields.items()}
+    with R.GpuSim(p) as sim:
+        sim.upload(other)
+        ref = sim.adjoint_step(lam)
+    with R.GpuSim(p) as sim:
+        sim.upload(st)
+        sim.adjoint_record(2, 1)
+        sim.upload(other)
+        with pytest.raises(R.R3dError) as e:
+            sim.adjoint_backward(lam)
+        assert e.value.code == R.R3D_ENUMERIC
+        got = sim.adjoint_step(lam)
+    for n in ref:
+        assert np.array_equal(got[n], ref[n]), n
