@@ -688,7 +688,11 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
                 rhs(EdgeTag<true>{});
             }
         }
-        if (SPLIT && s_abort) break;
+        if constexpr (SPLIT) {
+            // no CTA barrier orders this read against other warps' writes, so the warp decides as one: lanes
+            // that left alone would wait at the barrier below for those that wait for them at __syncwarp
+            if (__any_sync(0xffffffffu, *(volatile int*)&s_abort)) break;
+        }
         if constexpr (LEAN) {
             // hydro: the other rows' accumulators (prefetched into L2 a plane earlier), loaded after
             // the fluxes; the compiler barrier keeps the loads from being hoisted into them

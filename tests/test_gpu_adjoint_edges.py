@@ -46,7 +46,8 @@ def test_zero_safety_factor(extra):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("extra", [["--npx", "32", "--npy", "32", "--npz", "64"]], ids=["hydro"])
+@pytest.mark.parametrize("extra", [["--npx", "32", "--npy", "32", "--npz", "64"],
+                                   ["--npx", "24", "--npy", "20", "--npz", "40", *MAG]], ids=["hydro", "mhd"])
 def test_abandoned_recompute_leaves_nothing_behind(extra):
     """The recompute's bounded waits run out (single-wave stages, BCON planes in several chunks for hydro): the
     sweep reports it, and the forward steps, the sweeps and the trajectory after it are as without it."""

@@ -42,3 +42,41 @@ def test_bounded_tma_wait_reports_error_and_context_recovers(precision):
         sim.download(got)
     for n in ref.fields:
         assert np.array_equal(ref.fields[n], got.fields[n]), n
+
+
+MAG = ["--lmag", "1", "--beta", "10", "--rm", "1", "--ampb", "0.1", "--bfh", "2", "--bzp", "20"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,extra,launches", [
+    ((160, 96, 100), [], 9),
+    ((64, 32, 32), MAG, 4),    # 8-row tiles
+    ((64, 100, 96), MAG, 9),
+    ((64, 128, 128), MAG, 9),  # 6-row tiles
+    ((256, 256, 128), ["--precision", "fp32bulk"], 9),
+], ids=["hydro", "mhd8_single_wave", "mhd8", "mhd6", "fp32bulk"])
+def test_every_stage_form_reports_and_recovers(shape, extra, launches):
+    """The same in the other forms of the stages: launches of several waves (9 launches a step) and MHD, whose
+    plane barrier has an abort path of its own."""
+    flags = [f for n, v in zip(("--npx", "--npy", "--npz"), shape) for f in (n, str(v))]
+    p = R.parse(flags + ["--seed", "3"] + extra)
+    st = R.HostState.setup(p)
+    with R.GpuSim(p) as sim:
+        ref = st.copy()
+        sim.upload(st)
+        assert sim.run_timed(1)[1]["total_launches"] == launches
+        sim.download(ref)
+        for _ in range(2):
+            sim.debug_tma_extra(16)
+            t0 = time.time()
+            with pytest.raises(R.R3dError) as e:
+                sim.step()
+            assert e.value.code == R.R3D_ECUDA and "bounded TMA wait" in str(e.value)
+            assert time.time() - t0 < 30.0
+            sim.debug_tma_extra(0)
+            got = st.copy()
+            sim.upload(st)
+            sim.step()
+            sim.download(got)
+            for n in ref.fields:
+                assert np.array_equal(ref.fields[n], got.fields[n]), n
