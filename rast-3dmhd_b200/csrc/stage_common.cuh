@@ -58,17 +58,21 @@ __device__ __forceinline__ float dd2_est(double dd) {
 // takes s^2 = the Mach term's threshold, where the bound is tight).  So a cell has um < thr_um and
 // every limit above its threshold when |m|^2 < u T rho^2, dd^2 rho^2 > a1 |m|^2 + a2 T rho^2 +
 // a3 |B|^2 rho and dd^2 rho > max(q2 rkapa, q3) - products and sums of positive quantities, formed in
-// float from correctly rounded inputs in 2^-30 .. 2^30 with a relative error below 2^-19, against
-// coefficients that step_begin widens by 2^-10.  A non-finite value fails a comparison and the
-// cell is evaluated.  The folded limits over the whole domain are exact whenever the final minima
+// float from inputs in 2^-30 .. 2^30, against coefficients that step_begin widens by 2^-10.  From
+// correctly rounded inputs both sides have a relative error below 2^-19.  FP32-bulk forms rho and T as
+// float(background) + deviation, off by up to 2^-24 of the background and a rounding: where they are
+// 2^-8 of the background or more (rlo, tlo), 2^-16 relative, and 2^-13 over the two sides' five factors.
+// A non-finite value fails a comparison and the cell is evaluated.  The folded limits over the whole domain are exact whenever the final minima
 // are <= and the maximum >= their thresholds (checked by step_end, which requests a full
 // re-evaluation otherwise).  The resistive limit depends on the grid alone: the whole-state
 // evaluation after an upload leaves its minimum, which no step clears.
 // dd2: min(dd2_est(min(ddx, ddy)), dd2_est(ddz)); qk: max(q2 rkapa, q3); dd evaluates min_of3(...).
+// rlo, tlo: the smallest rho and T of the estimates.
+constexpr float kDtLow = 0x1p-30f;
 __device__ __forceinline__ bool dt_skip(const DtBounds& B, float ru, float rv, float rw, float ro, float tt,
-                                        float bcfl, float dd2, float qk) {
+                                        float bcfl, float dd2, float qk, float rlo = kDtLow, float tlo = kDtLow) {
     const float msq = ru * ru + rv * rv + rw * rw, r2 = ro * ro, tr2 = tt * r2;
-    return ro >= 0x1p-30f && ro < 0x1p30f && tt >= 0x1p-30f && tt < 0x1p30f && msq < B.u * tr2 &&
+    return ro >= rlo && ro < 0x1p30f && tt >= tlo && tt < 0x1p30f && msq < B.u * tr2 &&
            dd2 * r2 > B.a1 * msq + B.a2 * tr2 + bcfl && dd2 * ro > qk;
 }
 

@@ -404,13 +404,15 @@ __global__ void __launch_bounds__(Sh::NT, STAGE == 2 ? Sh::ctas_s2 : Sh::ctas)
         }
         if (STAGE == 2 && !edge) {  // dt limits: the filter in FP32, FP64 values on the full state
             const float dd2z = dd2_est(L.ddz[k]), qk = fmaxf(s_bnd.q2 * kb4.w, s_bnd.q3);
+            const float rbg = bg.rf[k], tbg = bg.tf[k];
+            const float rlo = fmaxf(kDtLow, 0x1p-8f * rbg), tlo = fmaxf(kDtLow, 0x1p-8f * tbg);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (h == 1 && !act1) break;
                 const float a0 = h ? xn[0].y : xn[0].x, a1 = h ? xn[1].y : xn[1].x, a2 = h ? xn[2].y : xn[2].x;
                 const float a3 = h ? xn[3].y : xn[3].x, a4 = h ? xn[4].y : xn[4].x;
-                const float rof = bg.rf[k] + a3, ttf = bg.tf[k] + a4;
-                if (!dt_skip(s_bnd, a0, a1, a2, rof, ttf, 0.0f, fminf(h ? dd21 : dd20, dd2z), qk)) {
+                const float rof = rbg + a3, ttf = tbg + a4;
+                if (!dt_skip(s_bnd, a0, a1, a2, rof, ttf, 0.0f, fminf(h ? dd21 : dd20, dd2z), qk, rlo, tlo)) {
                     double w1, w2, w3, w4, um;
                     const double dd = min_of3(L.ddx[i + h], L.ddy[j], L.ddz[k]);
                     const double ro = bg.r[k] + (double)a3, tt = bg.t[k] + (double)a4;

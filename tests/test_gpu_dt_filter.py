@@ -107,3 +107,42 @@ def test_slabs_filter_on_their_own_limits(margin):
         assert refolds == 6 * 3
     else:
         assert refolds <= 3
+
+
+@pytest.mark.gpu
+def test_fp32bulk_temperature_that_cancels_its_background():
+    """A cell at rest with its neighbours but for a small momentum, whose T is 2^-23 of the background: the
+    float sum background + deviation is off by several percent there.  It holds the largest Mach term, another
+    cell one 0.5% below it (inside the filter's margin): umach is the first one's, as without thresholds."""
+    flags = ["--npx", "40", "--npy", "24", "--npz", "32", "--ngrid", "0", "--precision", "fp32bulk",
+             "--sff", "1e-30", "--tp", "0"]  # steps too short to change a float
+    p = R.parse(flags)
+    t, r = R.static_profile(p)
+    tf = t.astype(np.float32)
+    ulp = np.spacing(tf).astype(float)
+    err = (tf.astype(float) - t) / ulp  # in (-0.5, 0.5): the sum is (1 - err) ulp, its float one ulp
+    k = 8 + int(np.argmax(err[8:-8]))
+    assert err[k] > 0.1
+    st = R.HostState.setup(p)
+    for n in ("ru", "rv", "rw"):
+        st.fields[n][...] = 0.0
+    tc = np.concatenate([t[:1], t, t[-1:]])
+    rc = np.concatenate([r[:1], r, r[-1:]])
+    st.fields["tt"][...] = tc[:, None, None]
+    st.fields["ro"][...] = rc[:, None, None]
+    tiny = float(tf[k] - np.float32(ulp[k])) * -1.0 + t[k]
+    st.fields["tt"][k + 1, 12, 20] = tiny
+    mach2 = 1e-4
+    for j, tt, m2 in ((12, tiny, mach2), (6, t[k], 0.995 * mach2)):
+        st.fields["ru"][k + 1, j, 20] = np.sqrt(m2 * p.gamma * tt) * r[k]
+    got = {}
+    for margin in (None, 1e30):
+        with R.GpuSim(p) as sim:
+            if margin is not None:
+                sim.debug_dt_filter(margin)
+            sim.upload(st)
+            sim.step()
+            sc = sim.step()  # its start holds the first step's limits
+            got[margin] = (sc["umach"], sc["dt"])
+    assert got[None] == got[1e30]
+    assert abs(got[None][0] / np.sqrt(mach2) - 1.0) < 1e-6
