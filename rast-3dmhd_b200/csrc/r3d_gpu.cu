@@ -14,6 +14,7 @@
 //    arrays to the host per step for dt, src/gpu.cpp:790-823).
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <cerrno>
@@ -405,10 +406,13 @@ struct Fp64Staging {
 };
 
 // The bounce buffers: 8 MB each, large enough that a chunk's device copy hides behind the host's (2 MB
-// chunks were 10% slower).  Page-locking costs about 1 ms per MB once per handle, so arrays below 4 MB
-// stay with the driver's own staging: there a first call would pay more than it saves.  B200, 16 host
-// cores: 128x128x128 adjoint_step (17.6 MB per field each way) 27.2 ms with the driver's staging, 12.6.
-constexpr size_t kBounce = size_t(8) << 20, kDirect = size_t(4) << 20;
+// chunks were 10% slower), made on first use, the second for arrays of several chunks only.  Of huge
+// pages, because a first call on a handle pays for them: page-locking 16 MB took 2.3 ms, as cudaMallocHost
+// 8 to 10 (first upload and download of 64x64x128 hydro 4.6 ms against 11, with the driver's staging 4.6;
+// 128x128x128 9.2 against 17 and 16).  Arrays below 4 MB stay with the driver's own staging: there a first
+// call would pay more than it saves.  B200, 16 host cores: 128x128x128 adjoint_step (17.6 MB per field each
+// way) 27.2 ms with the driver's staging, 12.6.
+constexpr size_t kBounce = size_t(8) << 20, kDirect = size_t(4) << 20, kHugePage = size_t(2) << 20;
 
 bool pageable(const void* p) {
     cudaPointerAttributes at{};
@@ -419,10 +423,25 @@ bool pageable(const void* p) {
     return at.type == cudaMemoryTypeUnregistered;
 }
 
-void bounce_ready(r3d_gpu* g) {
-    for (int s = 0; s < 2; ++s) {
-        if (!g->bounce[s]) cuda_ok(cudaMallocHost(&g->bounce[s], kBounce), "cudaMallocHost(copy buffer)");
+void bounce_ready(r3d_gpu* g, int count) {
+    for (int s = 0; s < count; ++s) {
+        if (g->bounce[s]) continue;
         if (!g->bounce_ev[s]) cuda_ok(cudaEventCreateWithFlags(&g->bounce_ev[s], cudaEventDisableTiming), "event");
+        void* p = std::aligned_alloc(kHugePage, kBounce);
+        if (!p) throw Error(R3D_ENOMEM, "no memory for a copy buffer");
+        madvise(p, kBounce, MADV_HUGEPAGE);
+        const cudaError_t e = cudaHostRegister(p, kBounce, cudaHostRegisterDefault);
+        if (e != cudaSuccess) std::free(p);
+        cuda_ok(e, "cudaHostRegister(copy buffer)");
+        g->bounce[s] = p;
+    }
+}
+
+void bounce_free(r3d_gpu* g) {
+    for (int s = 0; s < 2; ++s) {
+        if (g->bounce[s]) cudaHostUnregister(g->bounce[s]);
+        std::free(g->bounce[s]);
+        if (g->bounce_ev[s]) cudaEventDestroy(g->bounce_ev[s]);
     }
 }
 
@@ -432,8 +451,8 @@ void to_host(r3d_gpu* g, void* dst, const void* src, size_t pitch, size_t width,
         cuda_ok(cudaMemcpy2DAsync(dst, width, src, pitch, width, rows, cudaMemcpyDeviceToHost, g->stream), what);
         return;
     }
-    bounce_ready(g);
     const size_t n = (rows + per - 1) / per;
+    bounce_ready(g, n > 1 ? 2 : 1);
     for (size_t c = 0; c <= n; ++c) {  // chunk c into its buffer while chunk c - 1 goes on to dst
         if (c < n) {
             const size_t m = std::min(per, rows - c * per);
@@ -455,7 +474,7 @@ void from_host(r3d_gpu* g, void* dst, const void* src, size_t bytes, const char*
         cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, g->stream), what);
         return;
     }
-    bounce_ready(g);
+    bounce_ready(g, bytes > kBounce ? 2 : 1);
     for (size_t off = 0, c = 0; off < bytes; off += kBounce, ++c) {
         const size_t m = std::min(kBounce, bytes - off);
         // an event never recorded counts as complete
@@ -1083,10 +1102,7 @@ void destroy_handle(r3d_gpu* g) {
     cudaFree(g->dsc);
     cudaFree(g->edge_cnt);
     if (g->hsc) cudaFreeHost(g->hsc);
-    for (int s = 0; s < 2; ++s) {
-        if (g->bounce[s]) cudaFreeHost(g->bounce[s]);
-        if (g->bounce_ev[s]) cudaEventDestroy(g->bounce_ev[s]);
-    }
+    bounce_free(g);
     for (auto e : g->ev) cudaEventDestroy(e);
     if (g->stream && g->own_stream) cudaStreamDestroy(g->stream);
     delete g;
