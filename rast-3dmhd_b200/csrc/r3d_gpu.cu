@@ -423,18 +423,22 @@ bool pageable(const void* p) {
     return at.type == cudaMemoryTypeUnregistered;
 }
 
-void bounce_ready(r3d_gpu* g, int count) {
+// False where the host has no memory for them, or none to lock: the driver's staging needs none.
+bool bounce_ready(r3d_gpu* g, int count) {
     for (int s = 0; s < count; ++s) {
         if (g->bounce[s]) continue;
         if (!g->bounce_ev[s]) cuda_ok(cudaEventCreateWithFlags(&g->bounce_ev[s], cudaEventDisableTiming), "event");
         void* p = std::aligned_alloc(kHugePage, kBounce);
-        if (!p) throw Error(R3D_ENOMEM, "no memory for a copy buffer");
+        if (!p) return false;
         madvise(p, kBounce, MADV_HUGEPAGE);
-        const cudaError_t e = cudaHostRegister(p, kBounce, cudaHostRegisterDefault);
-        if (e != cudaSuccess) std::free(p);
-        cuda_ok(e, "cudaHostRegister(copy buffer)");
+        if (cudaHostRegister(p, kBounce, cudaHostRegisterDefault) != cudaSuccess) {
+            cudaGetLastError();
+            std::free(p);
+            return false;
+        }
         g->bounce[s] = p;
     }
+    return true;
 }
 
 void bounce_free(r3d_gpu* g) {
@@ -447,12 +451,11 @@ void bounce_free(r3d_gpu* g) {
 
 void to_host(r3d_gpu* g, void* dst, const void* src, size_t pitch, size_t width, size_t rows, const char* what) {
     const size_t per = kBounce / width;  // rows of a chunk
-    if (width * rows < kDirect || per == 0 || !pageable(dst)) {
+    if (width * rows < kDirect || per == 0 || !pageable(dst) || !bounce_ready(g, rows > per ? 2 : 1)) {
         cuda_ok(cudaMemcpy2DAsync(dst, width, src, pitch, width, rows, cudaMemcpyDeviceToHost, g->stream), what);
         return;
     }
     const size_t n = (rows + per - 1) / per;
-    bounce_ready(g, n > 1 ? 2 : 1);
     for (size_t c = 0; c <= n; ++c) {  // chunk c into its buffer while chunk c - 1 goes on to dst
         if (c < n) {
             const size_t m = std::min(per, rows - c * per);
@@ -470,11 +473,10 @@ void to_host(r3d_gpu* g, void* dst, const void* src, size_t pitch, size_t width,
 }
 
 void from_host(r3d_gpu* g, void* dst, const void* src, size_t bytes, const char* what) {
-    if (bytes < kDirect || !pageable(src)) {
+    if (bytes < kDirect || !pageable(src) || !bounce_ready(g, bytes > kBounce ? 2 : 1)) {
         cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, g->stream), what);
         return;
     }
-    bounce_ready(g, bytes > kBounce ? 2 : 1);
     for (size_t off = 0, c = 0; off < bytes; off += kBounce, ++c) {
         const size_t m = std::min(kBounce, bytes - off);
         // an event never recorded counts as complete
