@@ -56,7 +56,7 @@ def build(verbose_ptxas: bool = False, force: bool = False) -> str:
             extra = ["-Xptxas", "-v"] if (verbose_ptxas and s.endswith(".cu")) else []
             lang = ["-x", "cu"] if s.endswith(".cu") else ["-x", "c++"]
             fmad = ["-fmad=true"] if s in FMAD_ON else ["-fmad=false"]
-            omp = ["-Xcompiler", "-fopenmp"] if s in HOST_SRCS else []  # host set-up loops and copies
+            omp = ["-Xcompiler", "-fopenmp"] if s in HOST_SRCS else []  # host set-up loops
             _run([NVCC] + ARCH + COMMON + fmad + omp + extra + lang + ["-c", src, "-o", obj])
     if force or _stale(LIB, objs):
         _run([NVCC] + ARCH + ["-shared", "-Xcompiler", "-fPIC", "-o", LIB] + objs +

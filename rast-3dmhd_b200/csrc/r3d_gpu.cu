@@ -438,6 +438,7 @@ bool bounce_ready(r3d_gpu* g, int count) {
         }
         g->bounce[s] = p;
     }
+    if (!g->teams) g->teams = r3db::CopyTeams::get();
     return true;
 }
 
@@ -456,6 +457,8 @@ void to_host(r3d_gpu* g, void* dst, const void* src, size_t pitch, size_t width,
         return;
     }
     const size_t n = (rows + per - 1) / per;
+    r3db::CopyTeams::Use team(*g->teams);
+    team->wake();  // while the first chunk comes
     for (size_t c = 0; c <= n; ++c) {  // chunk c into its buffer while chunk c - 1 goes on to dst
         if (c < n) {
             const size_t m = std::min(per, rows - c * per);
@@ -467,7 +470,7 @@ void to_host(r3d_gpu* g, void* dst, const void* src, size_t pitch, size_t width,
         if (c > 0) {
             const size_t p = c - 1;
             cuda_ok(cudaEventSynchronize(g->bounce_ev[p & 1]), what);
-            r3db::parallel_copy((char*)dst + p * per * width, g->bounce[p & 1], std::min(per, rows - p * per) * width);
+            team->copy((char*)dst + p * per * width, g->bounce[p & 1], std::min(per, rows - p * per) * width);
         }
     }
 }
@@ -477,11 +480,12 @@ void from_host(r3d_gpu* g, void* dst, const void* src, size_t bytes, const char*
         cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, g->stream), what);
         return;
     }
+    r3db::CopyTeams::Use team(*g->teams);
     for (size_t off = 0, c = 0; off < bytes; off += kBounce, ++c) {
         const size_t m = std::min(kBounce, bytes - off);
         // an event never recorded counts as complete
         cuda_ok(cudaEventSynchronize(g->bounce_ev[c & 1]), what);
-        r3db::parallel_copy(g->bounce[c & 1], (const char*)src + off, m);
+        team->copy(g->bounce[c & 1], (const char*)src + off, m);
         cuda_ok(cudaMemcpyAsync((char*)dst + off, g->bounce[c & 1], m, cudaMemcpyHostToDevice, g->stream), what);
         cuda_ok(cudaEventRecord(g->bounce_ev[c & 1], g->stream), what);
     }

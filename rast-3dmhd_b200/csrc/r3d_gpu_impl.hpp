@@ -7,6 +7,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <utility>
 #include <vector>
@@ -76,6 +77,7 @@ struct r3d_gpu {
     int64_t steps_enqueued = 0;
     void* bounce[2] = {nullptr, nullptr};  // page-locked copy buffers (to_host, from_host)
     cudaEvent_t bounce_ev[2] = {nullptr, nullptr};
+    std::shared_ptr<r3db::CopyTeams> teams;  // their host side
 };
 
 namespace r3dg {

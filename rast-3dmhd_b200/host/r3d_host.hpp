@@ -8,6 +8,8 @@
 #pragma once
 
 #include <cstdint>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -97,7 +99,44 @@ void setup_state(const r3d_params& p, const r3d_host_state& st, r3d_scalars& sc,
 // domain: y rows first, then x columns).
 void fill_ghosts(double* f, int64_t nx, int64_t ny, int64_t nz);
 
-// memcpy by up to eight threads (hostcopy.cpp).
-void parallel_copy(void* dst, const void* src, size_t bytes);
+// memcpy by several threads (hostcopy.cpp): up to eight, no more than OMP_NUM_THREADS or the cores this
+// process may use, fewer where they cannot be made.  One copy at a time.
+class CopyTeam {
+  public:
+    CopyTeam();
+    ~CopyTeam();
+    CopyTeam(const CopyTeam&) = delete;
+    CopyTeam& operator=(const CopyTeam&) = delete;
+    void copy(void* dst, const void* src, size_t bytes);
+    void wake();  // a copy follows shortly
+    bool mine() const;  // its threads are this process's
+
+  private:
+    struct Shared;
+    Shared* s;
+};
+
+// The teams of a process, held by the handles that copy; the threads end with the last of them.  A transfer
+// takes a team for its duration, the one that was given back last (its threads may still be awake), so there
+// are as many as there have been transfers at once.
+class CopyTeams {
+  public:
+    static std::shared_ptr<CopyTeams> get();
+    class Use {
+      public:
+        explicit Use(CopyTeams& p);
+        ~Use();
+        CopyTeam* operator->() const { return team.get(); }
+
+      private:
+        CopyTeams& pool;
+        std::unique_ptr<CopyTeam> team;
+    };
+
+  private:
+    std::mutex m;
+    std::vector<std::unique_ptr<CopyTeam>> idle;  // has room for every team
+    size_t made = 0;
+};
 
 }  // namespace r3db

@@ -43,3 +43,29 @@ def test_copies_without_page_locked_buffers():
     """No address space is left for the buffers: the copies go through the driver's staging instead."""
     rc, out = child(NO_MEMORY)
     assert rc == 0 and "COPIED" in out, out
+
+
+FORKED = """
+import os, signal
+import numpy as np
+import r3d_b200 as R
+
+p = R.parse(["--npx", "64", "--npy", "64", "--npz", "120", "--seed", "5"])
+st = R.HostState.setup(p)  # OpenMP loops; CUDA not yet in use
+pid = os.fork()
+if pid == 0:
+    signal.alarm(120)
+    got = st.copy()
+    with R.GpuSim(p) as sim:
+        sim.upload(st)
+        sim.download(got)
+    os._exit(0 if all(np.array_equal(got.fields[n], st.fields[n]) for n in st.fields) else 1)
+assert os.waitpid(pid, 0)[1] == 0
+print("COPIED")
+"""
+
+
+@pytest.mark.gpu
+def test_copies_in_a_worker_forked_after_the_set_up():
+    rc, out = child(FORKED)
+    assert rc == 0 and "COPIED" in out, out
