@@ -676,7 +676,16 @@ void pull_scalars(r3d_gpu* g, r3d_scalars* sc) {
     take_scalars(g, sc);
 }
 
+// Whole steps that r3d_gpu_step runs eagerly, after create and after an upload that dropped the graphs,
+// before it captures them.  B200: the capture for a buffer parity takes 80 us at 32x32x64, 100 at MHD
+// 64x64x128 (0.6 ms the first of a process), two are needed, and a replay is 17 and 11 us shorter than an
+// eager step of 72 and 198.  Captured on the second and third step, those two and the first took 160, 140 and
+// 300 us where a program uploads, steps a few times and uploads again; the eager ones take 82, 70 and 210.
+// Four: more steps earn the captures back later, and a program that steps on loses 60 us.
+constexpr int64_t kEagerSteps = 4;
+
 void drop_graphs(r3d_gpu* g) {
+    g->single_steps = 0;
     for (auto* graphs : {g->step_graph, g->single_graph})
         for (int q = 0; q < 2; ++q) {
             if (graphs[q]) cudaGraphExecDestroy(graphs[q]);
@@ -1549,9 +1558,8 @@ int r3d_gpu_step(r3d_gpu* g, int nstages, r3d_scalars* sc) {
         if (!g->uploaded) throw Error(R3D_ESTATE, "step before upload");
         DeviceGuard dg(g->device);
         r3d_scalars tmp{};
-        if (nstages == 3 && g->steps_enqueued > 0 && graph_steps(g)) {
-            // one launch for the step and its read-back: at 32x32x64 the eager launches and the copy
-            // took 42 us per step beside 42 us of kernels
+        if (nstages == 3 && graph_steps(g) && (g->single_graph[g->cur] || g->single_steps >= kEagerSteps)) {
+            // one launch for the step and its read-back
             cudaGraphExec_t ex = captured_steps(g, g->single_graph, 1, true);
             cuda_ok(cudaGraphLaunch(ex, g->stream), "cudaGraphLaunch");
             g->cur = 1 - g->cur;  // three stages
@@ -1562,7 +1570,10 @@ int r3d_gpu_step(r3d_gpu* g, int nstages, r3d_scalars* sc) {
             Timer tm{g, false, nullptr};
             int a = 0, b = 0;
             enqueue_step(g, nstages, tm, a, b);
-            if (nstages == 3) ++g->steps_enqueued;
+            if (nstages == 3) {
+                ++g->steps_enqueued;
+                ++g->single_steps;
+            }
             pull_scalars(g, &tmp);
         }
         if (sc) *sc = tmp;

@@ -75,6 +75,7 @@ struct r3d_gpu {
     r3dk::Physics graph_ph{};   // the arguments the graphs were captured with that an upload may change
     r3dk::Boundary graph_bnd{};
     int64_t steps_enqueued = 0;
+    int64_t single_steps = 0;  // eager whole steps of r3d_gpu_step since the graphs were dropped
     void* bounce[2] = {nullptr, nullptr};  // page-locked copy buffers (to_host, from_host)
     cudaEvent_t bounce_ev[2] = {nullptr, nullptr};
     std::shared_ptr<r3db::CopyTeams> teams;  // their host side

@@ -4,9 +4,33 @@ import pytest
 
 import r3d_b200 as R
 
+# whole steps by r3d_gpu_step (the first four are eager), by r3d_gpu_run, and partial steps of one or two stages
+OPS = {
+    "step": [("step", 20)],
+    "mixed": [("step", 18), ("run", 3), ("partial", 2), ("step", 3), ("partial", 1), ("step", 3), ("run", 4)],
+    "run": [("run", 5)],
+    "few": [("step", 2)],
+}
+
 
 def same(a, b):
     return all(np.array_equal(a.fields[n], b.fields[n]) for n in a.fields)
+
+
+def session(sim, start, ops, eager=False):
+    sim.upload(start)
+    for kind, n in ops:
+        if kind == "partial":
+            sc = sim.step(n)
+        elif eager:  # a timed step is never a graph
+            sc = [sim.run_timed(1)[0] for _ in range(n)][-1]
+        elif kind == "step":
+            sc = [sim.step() for _ in range(n)][-1]
+        else:
+            sc = sim.run(n)
+    got = start.copy()
+    sim.download(got)
+    return got, sc
 
 
 @pytest.mark.gpu
@@ -21,28 +45,15 @@ def test_steps_graphs_and_reuploads(flags):
     other = st.copy()  # another bottom temperature and another conductivity profile
     other.scalars["tb"] = st.scalars["tb"] * 1.01
     other.lines["rkapa"] = 1.0 + 0.1 * np.linspace(0.0, 1.0, p.npz + 2)
-
-    def run(sim, start, how):
-        sim.upload(start)
-        if how == "step":
-            sc = [sim.step() for _ in range(5)][-1]
-        elif how == "mixed":  # graphs of both parities, a partial step between whole ones
-            sim.step()
-            sim.run(3)
-            sc = sim.step()
-        else:
-            sc = sim.run(5)
-        got = st.copy()
-        sim.download(got)
-        return got, sc
-
+    starts = {"st": st, "other": other}
     ref = {}
-    for name, start in (("st", st), ("other", other)):
-        with R.GpuSim(p) as sim:
-            ref[name] = run(sim, start, "run")
-    assert not same(ref["st"][0], ref["other"][0])
+    for how in OPS:
+        for name, start in starts.items():
+            with R.GpuSim(p) as sim:
+                ref[how, name] = session(sim, start, OPS[how], eager=True)
+        assert not same(ref[how, "st"][0], ref[how, "other"][0])
     with R.GpuSim(p) as sim:  # one handle through all of them
-        for how in ("step", "mixed", "run", "step"):
-            for name, start in (("st", st), ("other", other)):
-                got, sc = run(sim, start, how)
-                assert same(got, ref[name][0]) and sc == ref[name][1], (how, name)
+        for how in ("step", "mixed", "run", "few", "step"):
+            for name in ("st", "other", "other"):
+                got, sc = session(sim, starts[name], OPS[how])
+                assert same(got, ref[how, name][0]) and sc == ref[how, name][1], (how, name)
