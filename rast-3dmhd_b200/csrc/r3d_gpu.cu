@@ -279,6 +279,21 @@ int launch_depth(int64_t tiles, int nloc, int planned, int64_t slots) {
     return best;
 }
 
+// R3D_KCHUNK=<planes> overrides the z-chunk depth of the stage kernels (tuning): a whole decimal
+// number, clamped to [1, nloc]; anything else is ignored (0), with a note on stderr if asked for.
+int chunk_override(int nloc, bool note) {
+    const char* e = getenv("R3D_KCHUNK");
+    if (!e) return 0;
+    char* end = nullptr;
+    errno = 0;
+    const long v = strtol(e, &end, 10);
+    if (end == e || *end != '\0' || errno == ERANGE || v < 1) {
+        if (note) fprintf(stderr, "r3d: R3D_KCHUNK='%s' is not a positive whole number; ignored\n", e);
+        return 0;
+    }
+    return (int)std::min<long>(v, nloc);
+}
+
 // z-chunk depth (planes per CTA) of the stage kernels of a handle over nloc local planes, given
 // its precision, FP64 column-tile rows and the device's SM count; R3D_KCHUNK=<planes> in the
 // environment overrides it.
@@ -314,19 +329,9 @@ int stage_chunk_depth(const r3d_params& p, bool fp32, int tile_rows, int nloc, i
             depth = plan_chunk_depth(tiles, nloc, depth, slots);
         }
     }
-    // R3D_KCHUNK=<planes> overrides the z-chunk depth of the stage kernels (tuning): a whole
-    // decimal number, clamped to [1, nloc]; anything else is ignored with a note on stderr
-    if (const char* e = getenv("R3D_KCHUNK")) {
-        char* end = nullptr;
-        errno = 0;
-        const long v = strtol(e, &end, 10);
-        if (end == e || *end != '\0' || errno == ERANGE || v < 1) {
-            fprintf(stderr, "r3d: R3D_KCHUNK='%s' is not a positive whole number; ignored\n", e);
-        } else {
-            const int k = (int)std::min<long>(v, nloc);
-            if (k != depth) fprintf(stderr, "r3d: R3D_KCHUNK overrides the z-chunk depth: %d planes (planned %d)\n", k, depth);
-            depth = k;
-        }
+    if (const int k = chunk_override(nloc, true)) {
+        if (k != depth) fprintf(stderr, "r3d: R3D_KCHUNK overrides the z-chunk depth: %d planes (planned %d)\n", k, depth);
+        depth = k;
     }
     return depth;
 }
@@ -1079,7 +1084,8 @@ r3d_gpu* create_handle(const r3d_params& pin, int z0, int nloc, cudaStream_t sha
                 const int64_t tiles = (int64_t)((p->npx + 31) / 32) * ((p->npy + rows - 1) / rows);
                 const int64_t slots = (int64_t)g->num_sms * (g->fp32 ? r3dk::stage_fp32_ctas_per_sm()
                                                                      : r3dk::stage_fp64_ctas_per_sm(p->lmag, rows));
-                g->depth = (p->lmag || getenv("R3D_KCHUNK")) ? g->kchunk : launch_depth(tiles, nloc, g->kchunk, slots);
+                g->depth = (p->lmag || chunk_override(nloc, false)) ? g->kchunk
+                                                                    : launch_depth(tiles, nloc, g->kchunk, slots);
                 g->ph.id_mode = p->id;
                 // launches of at most one wave take the single-wave form
                 g->tail = tiles * ((nloc + g->depth - 1) / g->depth) <= slots &&

@@ -121,3 +121,17 @@ def test_pageable_and_page_locked_arrays(shape, precision):
         assert np.array_equal(a, out["locked"][n]), n
     for n in out["pageable"]:
         assert np.isfinite(out["pageable"][n]).all(), n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value,launches", [(None, 9), ("sixteen", 9), ("0", 9), ("16", 4)])
+def test_depth_override(value, launches, monkeypatch):
+    """160x96x100: the planned 16 planes per CTA are one wave (4 launches a step), which a handle cuts into several
+    (9).  R3D_KCHUNK is taken as it is; what is ignored leaves the cut."""
+    monkeypatch.delenv("R3D_KCHUNK", raising=False)
+    if value is not None:
+        monkeypatch.setenv("R3D_KCHUNK", value)
+    p = R.parse(grid(160, 96, 100))
+    with R.GpuSim(p) as sim:
+        sim.setup()
+        assert sim.run_timed(1)[1]["total_launches"] == launches
