@@ -618,7 +618,7 @@ int r3d_gpu_adjoint_memory(const r3d_gpu* g, int64_t* bytes) {
         int64_t b = 0;
         if (A) {
             const int64_t st = (int64_t)A->nf * A->field_elems * (int64_t)sizeof(double);
-            b = A->bytes + st * (int64_t)(A->ckpt.size() + A->seg.size());
+            b = A->bytes + st * (int64_t)(A->ckpt.size() + A->seg.size()) + A->lim_steps * (int64_t)sizeof(g->dsc->wmin);
         }
         *bytes = b;
     });

@@ -102,3 +102,15 @@ def test_diverged_recompute_is_reported_once():
         got = sim.adjoint_step(lam)
     for n in ref:
         assert np.array_equal(got[n], ref[n]), n
+
+
+@pytest.mark.gpu
+def test_memory_counts_the_recorded_limits():
+    p = R.parse(["--npx", "16", "--npy", "12", "--npz", "16", "--seed", "3"])
+    got = []
+    for steps in (4, 40):
+        with R.GpuSim(p) as sim:
+            sim.setup()
+            sim.adjoint_record(steps, steps)  # two checkpoints
+            got.append(sim.adjoint_memory_bytes)
+    assert got[1] - got[0] == 36 * 32
