@@ -73,7 +73,8 @@ typedef struct r3d_host_state {
 typedef struct r3d_timing {
     double total_ms;        /* whole run, first launch to last */
     double stage_ms;        /* sum over the fused stage kernels */
-    double bcon_ms;         /* sum over BCON + ghost + dt-edge kernels */
+    double bcon_ms;         /* sum over BCON + ghost + dt-edge kernels: 0 where the stage launches are a
+                             * single wave, whose stages do this themselves */
     double other_ms;        /* dt finalise / scalar kernels */
     int stage_launches;
     int total_launches;     /* kernels launched by the library in the run */
@@ -182,9 +183,9 @@ int r3d_gpu_download_work(r3d_gpu* g, double* const* out);
  * usable.  0 (the default, restored by r3d_gpu_upload) switches it off. */
 int r3d_gpu_debug_tma_extra(r3d_gpu* g, unsigned int bytes);
 
-/* The third stage's time-step limits are folded through a filter: cells whose float estimates
- * of the CFL limit and Mach term lie clearly beyond the previous step's limits widened by a
- * relative margin (default 1/64) skip the exact FP64 evaluation, and when the folded result
+/* The third stage's time-step limits are folded through a filter: cells whose CFL, conduction and
+ * viscosity limits and Mach term, bounded in float, all lie clearly beyond the previous step's widened by
+ * a relative margin (default 1/64) skip the exact FP64 evaluation, and when the folded result
  * fails the check that makes this exact, the limits are evaluated again over the whole state
  * (a "refold").  The dt is bit-identical either way.  Test hook: margin (NaN: unchanged) sets
  * the margin - a negative one makes every full step refold - and *refolds (may be NULL)
@@ -196,7 +197,8 @@ int r3d_gpu_debug_dt_filter(r3d_gpu* g, double margin, int* refolds);
 
 /* Launch plan of the stage kernels for a handle created with *p over nloc local z planes (0:
  * the whole npz, as r3d_gpu_create) on a device with num_sms multiprocessors: *kchunk receives
- * the z planes each CTA marches through, *tile_rows the rows of its 32-column tile.  With
+ * the planned z planes per CTA (a hydro handle may use fewer, see below), *tile_rows the rows of its
+ * 32-column tile.  With
  * num_sms > 0 this is host-only (no device needed); num_sms <= 0 reads the SM count of device
  * p->gpu_id, as a handle does at create.  R3D_KCHUNK=<planes> in the environment (a whole
  * number, clamped to [1, nloc]) overrides the depth, as it does for a handle.  The depth starts at 64

@@ -46,7 +46,6 @@ struct Physics {
     // + d2z(rho - rom) * dv_ore*wwz, rom the horizontal mean of rho per plane
     int id_mode;
     double id_dh, id_dv, id_dh_ore, id_dv_ore;  // DH, DV and DH*ORE, DV*ORE
-    float gamma_f, ogamma_f, obeta_f;  // float copies for the estimates of the dt filter
 };
 
 // 1D metric tables (device pointers).

@@ -1062,7 +1062,6 @@ r3d_gpu* create_handle(const r3d_params& pin, int z0, int nloc, cudaStream_t sha
             for (int s = 0; s < 3; ++s) { ph.gam[s] = d.gam[s]; ph.zeta[s] = d.zeta[s]; }
             ph.lrot = p->lrot; ph.lmag = p->lmag;
             ph.kappa_const = 1;
-            ph.gamma_f = (float)ph.gamma; ph.ogamma_f = (float)ph.ogamma; ph.obeta_f = (float)ph.obeta;
             r3dk::Boundary& b = g->bnd;
             // 3dmhdsub.f:2807-2887: a plume for itcon 0/1 with tp != 0, else constant T for itcon
             // 0 and 2 (the latter with the embedded heat loss in FLUXES), half-domain T for 4,

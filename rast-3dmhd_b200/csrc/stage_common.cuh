@@ -33,8 +33,8 @@ __device__ __forceinline__ void dt_terms(const Physics& ph, double ru, double rv
 }
 
 // std::min(acc, v) / std::max(acc, v): a NaN v never replaces acc.
-__device__ __forceinline__ double fold_min(double acc, double v);
-__device__ __forceinline__ double fold_max(double acc, double v);
+__device__ __forceinline__ double fold_min(double acc, double v) { return (v < acc) ? v : acc; }
+__device__ __forceinline__ double fold_max(double acc, double v) { return (acc < v) ? v : acc; }
 
 // True when x is positive and 2^-30 <= x < 2^31 (one integer compare on the high word): the
 // window in which the float estimates below keep their error bound.
@@ -96,9 +96,6 @@ __device__ __forceinline__ double min_of3(double a, double b, double c) {
     const double m = (b < a) ? b : a;
     return (c < m) ? c : m;
 }
-// std::min(acc, v) / std::max(acc, v): a NaN v never replaces acc.
-__device__ __forceinline__ double fold_min(double acc, double v) { return (v < acc) ? v : acc; }
-__device__ __forceinline__ double fold_max(double acc, double v) { return (acc < v) ? v : acc; }
 
 // The limit that sets dt, chosen from the four minima's keys as step_begin_kernel does: 0 CFL,
 // 1 conduction, 2 viscosity, 3 resistivity; m receives its value.
