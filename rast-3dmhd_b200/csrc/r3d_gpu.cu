@@ -428,17 +428,30 @@ bool pageable(const void* p) {
     return at.type == cudaMemoryTypeUnregistered;
 }
 
+// Kept out of forked children: a page that a child shares would be copied on its next write here, away
+// from the one the device knows.
+void* huge_pages(size_t bytes) {
+    void* m = mmap(nullptr, bytes + kHugePage, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (m == MAP_FAILED) return nullptr;
+    char* b = static_cast<char*>(m);
+    const size_t head = (kHugePage - reinterpret_cast<uintptr_t>(b) % kHugePage) % kHugePage;
+    if (head) munmap(b, head);
+    munmap(b + head + bytes, kHugePage - head);
+    madvise(b + head, bytes, MADV_HUGEPAGE);
+    madvise(b + head, bytes, MADV_DONTFORK);
+    return b + head;
+}
+
 // False where the host has no memory for them, or none to lock: the driver's staging needs none.
 bool bounce_ready(r3d_gpu* g, int count) {
     for (int s = 0; s < count; ++s) {
         if (g->bounce[s]) continue;
         if (!g->bounce_ev[s]) cuda_ok(cudaEventCreateWithFlags(&g->bounce_ev[s], cudaEventDisableTiming), "event");
-        void* p = std::aligned_alloc(kHugePage, kBounce);
+        void* p = huge_pages(kBounce);
         if (!p) return false;
-        madvise(p, kBounce, MADV_HUGEPAGE);
         if (cudaHostRegister(p, kBounce, cudaHostRegisterDefault) != cudaSuccess) {
             cudaGetLastError();
-            std::free(p);
+            munmap(p, kBounce);
             return false;
         }
         g->bounce[s] = p;
@@ -449,8 +462,10 @@ bool bounce_ready(r3d_gpu* g, int count) {
 
 void bounce_free(r3d_gpu* g) {
     for (int s = 0; s < 2; ++s) {
-        if (g->bounce[s]) cudaHostUnregister(g->bounce[s]);
-        std::free(g->bounce[s]);
+        if (g->bounce[s]) {
+            cudaHostUnregister(g->bounce[s]);
+            munmap(g->bounce[s], kBounce);
+        }
         if (g->bounce_ev[s]) cudaEventDestroy(g->bounce_ev[s]);
     }
 }

@@ -69,3 +69,33 @@ print("COPIED")
 def test_copies_in_a_worker_forked_after_the_set_up():
     rc, out = child(FORKED)
     assert rc == 0 and "COPIED" in out, out
+
+
+CHILDREN = """
+import os, time
+import numpy as np
+import r3d_b200 as R
+
+p = R.parse(["--npx", "64", "--npy", "64", "--npz", "300", "--seed", "5"])  # 10.5 MB per field: both buffers
+st = R.HostState.setup(p)
+got = st.copy()
+with R.GpuSim(p) as sim:
+    for turn in range(3):
+        for n in st.fields:
+            st.fields[n] += 1.0
+        sim.upload(st)
+        pid = os.fork()  # alive through the next copies, which rewrite the buffers
+        if pid == 0:
+            time.sleep(0.5)
+            os._exit(0)
+        sim.download(got)
+        assert all(np.array_equal(got.fields[n], st.fields[n]) for n in st.fields), turn
+        os.waitpid(pid, 0)
+print("COPIED")
+"""
+
+
+@pytest.mark.gpu
+def test_copies_beside_a_forked_child():
+    rc, out = child(CHILDREN)
+    assert rc == 0 and "COPIED" in out, out
