@@ -82,10 +82,9 @@ __global__ void __launch_bounds__(BX* BY) adj_bcon_kernel(r3dk::Geometry g, r3dk
 
 // Bound by the latency of the gathers, so by how many loads the warps of an SM keep in flight: two
 // 256-thread blocks per SM (three for hydro pass 1) with every load of a cell free to go out at once.
-// B200, us per stage, while lambda_Y was still added by pass 1 and pass 2 did not prefetch:
-// 128x128x128 hydro pass 1 154 (two blocks: 165), pass 2 170 (three blocks, 80 registers and spills:
-// 192); 64x64x128 MHD pass 1 69 (three: 77), pass 2 87 (three: 97).  Now 150 + 152 and 65 + 95.  The
-// passes they replace, which stored every Lambda and folded lambda_F separately: 577 and 222.
+// B200, us per stage: 128x128x128 hydro pass 1 145 (two blocks: 173), pass 2 160 (three blocks, 80
+// registers and spills: 210); 64x64x128 MHD pass 1 65 (three: 77), pass 2 91 (three: 116).  Both
+// together, with every Lambda stored and lambda_F folded separately: 577 and 222.
 template <bool MHD>
 __global__ void __launch_bounds__(BX* BY, MHD ? 2 : 3) adj_pass1_kernel(const __grid_constant__ AdjArgs A, double* dots) {
     const int i = 1 + blockIdx.x * BX + threadIdx.x;
@@ -97,9 +96,10 @@ __global__ void __launch_bounds__(BX* BY, MHD ? 2 : 3) adj_pass1_kernel(const __
 }
 
 // The cell of this thread in the block `ahead` places later in launch order (-1: none): with as many
-// places as blocks run at once, its lines are in L2 by the time that block gathers them (pass 2,
-// 128x128x128 hydro 170 -> 143 us, 64x64x128 MHD 87 -> 84, both before it also read lambda_Y; twice as
-// far ahead 151 and 96.  Pass 1, whose gathers are fewer, was 5% slower with it).
+// places as blocks run at once, its lines are in L2 by the time that block gathers them.  B200, 128x128x128
+// hydro pass 2 181 -> 160 us (twice as far ahead 181); a whole step of the sweep 1674 -> 1616 us, at
+// 200x200x100 3137 -> 2975, MHD 126x126x128 2577 -> 2553, 64x64x128 820 -> 837.  Pass 1, whose gathers are
+// fewer, was 5% slower with it.
 __device__ __forceinline__ int cell_ahead(const r3dk::Geometry& g, int ahead) {
     const int b = block_linear() + ahead, row = b / (int)gridDim.x;
     const int i = 1 + (b % (int)gridDim.x) * BX + threadIdx.x;
@@ -451,8 +451,7 @@ void compare_states(r3d_gpu* g, Adjoint* A, const double* a, const double* b) {
 
 // Host cotangent (NX*NY*NZ per field, ghosts included) -> lam: x/y ghost entries are added to
 // the interior cells they image, z ghost planes are constants and dropped.  The fields pass through
-// F[0], which holds nothing between steps.  (Folding on the host, cell by cell, and copying the
-// gradient back the same way took 60 of the 64 ms of a 128x128x128 hydro adjoint_step.)
+// F[0], which holds nothing between steps.
 void upload_seed(r3d_gpu* g, Adjoint* A, const double* const* seed) {
     for (int f = 0; f < A->nf; ++f)
         if (!seed[f]) throw std::invalid_argument("null seed field");

@@ -21,13 +21,11 @@
 //     coef(m+e)*Lambda(m+e) to f's adjoint at m).  Every Lambda not stored is a product of values
 //     at one point - lambda_F times u, v, w, 1/rho, B - and is formed where it is gathered; the
 //     cross differences of the viscous stress are corner stencils of lambda_F itself.  lambda_Y, the
-//     largest term, is added last: added in pass 1 it was rounded again with every term that followed
-//     (128x128x128 hydro vjp, error against 64-bit torch 1.4e-16; 2.9e-17 so).
+//     largest term, is added last, so that it is rounded once (128x128x128 hydro vjp, error against
+//     64-bit torch 2.9e-17; added in pass 1 1.4e-16).
 //
-// Bound: the latency of the gathers, then DRAM.  One stage moves 106 arrays (MHD) where the form that
-// stored all 33 Lambda arrays and folded lambda_F in a pass of its own moved 146; splitting the
-// partials off pass 2 keeps it at 128 registers (with them it needed 174 and ran at 8 warps
-// per SM: 200 us at 64x64x128 MHD against 87).
+// Bound: the latency of the gathers, then DRAM: one stage moves 106 arrays with MHD, 67 without.  The
+// partials in pass 1 keep pass 2 at 128 registers (with them it needs 174 and runs 8 warps per SM).
 //
 // x and y are periodic: the forward reads ghost cells that are exact images of interior cells,
 // so the adjoint works on the npx x npy torus with wrapped neighbour indices and never stores an

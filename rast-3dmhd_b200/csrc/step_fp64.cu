@@ -72,7 +72,7 @@ constexpr int NDER = 4;
 // where it is used, the product the reference stores).  MHD keeps the 4-slot raw ring and the
 // derived u, v, w, P, 1/rho.  Both prefetch the RK accumulators of the next plane into L2 and
 // load a plane's accumulators during the plane - hydro the first row's before its fluxes and the
-// second row's after them, just before the stage update (504x504x128 on B200: 3826 -> 3804 us per step
+// second row's after them, just before the stage update (504x504x128 on B200: 3988 -> 3966 us per step
 // against both rows after; both before would spill), MHD before its derive phase - which takes fewer registers than holding the next
 // plane's values in registers (hydro: 40, and no spills).  Measured on B200 at 1965 MHz:
 // 504x504x512 hydro 15.45 -> 14.9 ms per step, 126x126x256 MHD 0.946 -> 0.901 ms (0.936 with
@@ -183,9 +183,9 @@ __global__ void __launch_bounds__(Cells<MHD, STAGE, TYV>::nt, Cells<MHD, STAGE, 
     constexpr bool LEAN = Ring<MHD>::lean;
     // MHD: the plane barrier in two halves.  A warp arrives when it has derived its part of plane k+1
     // and waits only before it first reads planes k+1 and k-1, after the velocity differences within
-    // plane k: with two CTAs per SM a whole barrier cost 0.9 of 6 cycles per issue (126x126x256 on
-    // B200, per step: 829 -> 818 us; with the field differences ahead of the wait too, which spills,
-    // 860).  Hydro (three CTAs per SM) was 1.5% slower with it, the FP32-bulk stage 11%.
+    // plane k: with two CTAs per SM a whole barrier cost 0.9 of 6 cycles per issue (B200, per step,
+    // 126x126x256: 834 -> 817 us, 252x252x256: 3190 -> 3151; with the field differences ahead of the
+    // wait too, which spills, 860).  Hydro (three CTAs per SM) was 1.5% slower with it, FP32-bulk 11%.
     constexpr bool SPLIT = MHD;
     // hydro: rows of the thread whose accumulators are loaded before the fluxes, the others after
     constexpr int ZE = (LEAN && STAGE > 0 && CPT > 1) ? 1 : 0;
