@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(BX* BY, MHD ? 2 : 3) adj_pass1_kernel(const __
 // The cell of this thread in the block `ahead` places later in launch order (-1: none): with as many
 // places as blocks run at once, its lines are in L2 by the time that block gathers them.  B200, 128x128x128
 // hydro pass 2 181 -> 160 us (twice as far ahead 181); a whole step of the sweep 1674 -> 1616 us, at
-// 200x200x100 3137 -> 2975, MHD 126x126x128 2577 -> 2553, 64x64x128 820 -> 837.  Pass 1, whose gathers are
-// fewer, was 5% slower with it.
+// 200x200x100 3137 -> 2975.  Not with MHD (64x64x128 pass 2 82 -> 91 us, a step 820 -> 837; 126x126x128 2577
+// -> 2553) nor in pass 1, whose gathers are fewer (5% slower).
 __device__ __forceinline__ int cell_ahead(const r3dk::Geometry& g, int ahead) {
     const int b = block_linear() + ahead, row = b / (int)gridDim.x;
     const int i = 1 + (b % (int)gridDim.x) * BX + threadIdx.x;
@@ -110,16 +110,18 @@ __device__ __forceinline__ int cell_ahead(const r3dk::Geometry& g, int ahead) {
 
 template <bool MHD>
 __global__ void __launch_bounds__(BX* BY, 2) adj_pass2_kernel(const __grid_constant__ AdjArgs A) {
-    if (const int n = cell_ahead(A.g, A.ahead); n >= 0) {
+    if constexpr (!MHD) {
+        if (const int n = cell_ahead(A.g, A.ahead); n >= 0) {
 #pragma unroll
-        for (int f = 0; f < (MHD ? 8 : 5); ++f) {
-            r3dk::prefetch_l2(A.x + f * A.fe + n);
-            r3dk::prefetch_l2(A.a + f * A.fe + n);
-            r3dk::prefetch_l2(A.out + f * A.fe + n);
-            r3dk::prefetch_l2(A.lam + f * A.fe + n);
+            for (int f = 0; f < 5; ++f) {
+                r3dk::prefetch_l2(A.x + f * A.fe + n);
+                r3dk::prefetch_l2(A.a + f * A.fe + n);
+                r3dk::prefetch_l2(A.out + f * A.fe + n);
+                r3dk::prefetch_l2(A.lam + f * A.fe + n);
+            }
+#pragma unroll
+            for (int q = 0; q < r3dk::kMidHydro; ++q) r3dk::prefetch_l2(A.mid + q * A.fe + n);
         }
-#pragma unroll
-        for (int q = 0; q < (MHD ? r3dk::kMidMax : r3dk::kMidHydro); ++q) r3dk::prefetch_l2(A.mid + q * A.fe + n);
     }
     const int i = 1 + blockIdx.x * BX + threadIdx.x;
     const int j = 1 + blockIdx.y * BY + threadIdx.y;
